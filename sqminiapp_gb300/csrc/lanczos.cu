@@ -177,7 +177,12 @@ cudaError_t launch_veff_extend(const double *veff, double vconst, void *ext, int
     const long long total = (long long)veff_quad_floats(p);
     const int block = 256;
     const int grid = (int)std::min<long long>((total + block - 1) / block, 152LL * 16);
-    veff_quad_kernel<<<grid, block, 0, s>>>(veff, vconst, p.cdiag, (float *)ext, p.Nx, p.Ny, p.Nz,
+    // the diagonal also takes up what the FP32 stencil weights lose on a constant vector, so
+    // that their rounding does not shift the low end of the spectrum
+    double diag = p.cdiag;
+    for (int d = 1; d <= kStencilHalf; d++)
+      diag += 2.0 * ((p.cx[d] - p.cxf[d]) + (p.cy[d] - p.cyf[d]) + (p.cz[d] - p.czf[d]));
+    veff_quad_kernel<<<grid, block, 0, s>>>(veff, vconst, diag, (float *)ext, p.Nx, p.Ny, p.Nz,
                                             p.nhx, p.nhy, p.nhz, p.EX, p.EY, p.EZ, p.vq_row);
     return cudaGetLastError();
   }

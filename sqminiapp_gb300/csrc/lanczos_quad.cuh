@@ -17,9 +17,9 @@
 //           13-plane register ring (one float4 load per plane); the x neighbours of the quad
 //           are four aligned float4 loads of the same row; it adds the diagonal (cdiag + Veff,
 //           read as one aligned float4 from a quad-aligned copy of the padded potential) and
-//           forms U <- (diag + Dz + Dx) v - b U;
+//           forms U <- s (diag + Dz + Dx) P - gamma U;
 //   pass B  a thread owns one quad of plane z over a y-range and walks y with a 13-row
-//           register ring: U += Dy v.
+//           register ring: U += s Dy P.
 // Eight consecutive threads own the quads of one row (pass A) or one plane (pass B), so a
 // quarter-warp's float4 accesses cover one contiguous row: no bank conflicts.
 //
@@ -28,10 +28,10 @@
 // it); consecutive lanes stream consecutive points, so every record load of a warp is one
 // contiguous 512-byte run.
 //
-// Per Lanczos step (P = b v_k unnormalised, U = v_{k-1}), four CTA barriers:
+// Per Lanczos step (v_k = s_k P with s_k a power of two, U = v_{k-1}), four CTA barriers:
 //   1  projector gather c = chi^T P (per-warp ranges of the node's list, one partial per
 //      warp and image, no atomics)  ||  pass A
-//   2  pass B  ||  alpha = Gamma c / b (and <v, V_nl v>)  -> per-warp partials of a_k
+//   2  pass B  ||  alpha = Gamma s c (and <P, V_nl P>)  -> per-warp partials of <P, H P>
 //   3  projector scatter U += chi alpha  ||  every warp reduces the a_k partials
 //   4  w = U - a_k v, P <- w, U <- v  -> per-warp partials of b_k^2
 // After barrier 4 every warp reduces the b partials itself (the same tree in every warp, so
@@ -41,10 +41,17 @@
 // FP64 pipe runs at a small fraction of its FP32 rate, so the step loop keeps FP64 out of its
 // critical path and converts to double only to store a_k and b_k.
 //
-// Memory traffic.  In the 12-warp budget pass A reads Veff through a per-thread ring of four
-// float4 in shared memory, filled by cp.async three planes ahead (slot-major: each warp access
-// is 512 contiguous bytes).  The list's stores and loads carry an L2 evict-last policy.  Nodes
-// after the first round come from a device-side queue.
+// Scaling.  The vector is never normalised: v_k = s_k P_k with s_k the power of two that brings
+// |v_k| into [1, 2), so no element is rounded by the scaling, and
+//   a_k = <P,HP> / |P|^2,   w = H v_k - a_k v_k - gamma_k v_{k-1},   P <- w,
+//   b_k = |w| / |v_k|,      gamma_{k+1} = s_{k+1} |w|^2 / |v_k|^2
+// with a_k and gamma_k as double-floats (head and tail applied).  Normalising by a rounded 1/b_k left
+// |v_k| off by 1e-7 and so a_k by twice that of its 18 + V: that, not the stencil's rounding, was
+// most of the FP32 error (weights 6e-6 -> 4e-7 and the lowest Ritz value 5e-7 -> 5e-8 Ha on a 27^3
+// cube without projectors, the diagonal's share of the weights' rounding included).
+//
+// Memory traffic.  Pass A reads Veff from L2 two planes ahead.  The list's stores and loads carry
+// an L2 evict-last policy.  Nodes after the first round come from a device-side queue.
 //
 // CTA pair (PAIR, lanczos_quad_pair_kernel): one node per cluster of two CTAs for cubes whose
 // P and U do not fit one CTA.  The cube is split in z (PairPlanes); each CTA owns its planes of
@@ -91,6 +98,51 @@ __device__ __forceinline__ float2 lo(float4 v) { return make_float2(v.x, v.y); }
 __device__ __forceinline__ float2 hi(float4 v) { return make_float2(v.z, v.w); }
 __device__ __forceinline__ float2 splat(float c) { return make_float2(c, c); }
 
+// Shared memory by byte address (cvta_shared): whole quads, and loads that a lane may skip (the
+// registers keep their values).  As C++ expressions the skipped loads of the stencil passes
+// became real branches, and the moves around them a third of all issued instructions.
+__device__ __forceinline__ unsigned smem_addr(const void *p) {
+  return (unsigned)__cvta_generic_to_shared(p);
+}
+__device__ __forceinline__ float4 lds_quad(unsigned a) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(a)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ void lds_quad_if(bool on, unsigned a, float4 &v) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %5, 0;\n\t@p ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+      : "+f"(v.x), "+f"(v.y), "+f"(v.z), "+f"(v.w)
+      : "r"(a), "r"((int)on)
+      : "memory");
+}
+__device__ __forceinline__ void lds_pair_if(bool on, unsigned a, float2 &v) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %3, 0;\n\t@p ld.shared.v2.f32 {%0, %1}, [%2];\n\t}"
+      : "+f"(v.x), "+f"(v.y)
+      : "r"(a), "r"((int)on)
+      : "memory");
+}
+__device__ __forceinline__ void sts_quad_if(bool on, unsigned a, float4 v) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %5, 0;\n\t@p st.shared.v4.f32 [%4], {%0, %1, %2, %3};\n\t}" ::"f"(v.x),
+      "f"(v.y), "f"(v.z), "f"(v.w), "r"(a), "r"((int)on)
+      : "memory");
+}
+// a quad of global memory, or zeros
+__device__ __forceinline__ float4 ldg_quad_if(bool on, const float4 *g) {
+  float4 v;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %5, 0;\n\tmov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\t"
+      "mov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t@p ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+      : "=&f"(v.x), "=&f"(v.y), "=&f"(v.z), "=&f"(v.w)
+      : "l"(g), "r"((int)on));
+  return v;
+}
+
 // Kahan-compensated FP32 running sum.
 struct Kahan {
   float s = 0.f, c = 0.f;
@@ -128,6 +180,17 @@ __device__ __forceinline__ DF df_warp_sum(DF v) {  // the same butterfly in ever
     v = df_add(v, w);
   }
   return v;
+}
+// Quotient of two double-floats as a double-float (relative error about 2^-45).
+__device__ __forceinline__ DF df_div(DF x, DF y) {
+  const float q = x.hi / y.hi;
+  const float r = fmaf(-q, y.hi, x.hi) + (x.lo - q * y.lo);
+  return DF{q, r / y.hi};
+}
+// The power of two s with s^2 n in [1, 4) (n a normal number above zero).
+__device__ __forceinline__ float unit_scale(float n) {
+  const int e = ((__float_as_int(n) >> 23) & 255) - 127;
+  return __int_as_float((127 - (e >> 1)) << 23);
 }
 // Sum of nw per-warp partials red[0..nw), the same tree in every lane of every warp, so every
 // thread gets the bit-identical total.
@@ -258,10 +321,11 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
   float *P = reinterpret_cast<float *>(smem_raw);
   float *U = P + ncp;
   unsigned char *cur = reinterpret_cast<unsigned char *>(U + ncu);
-  double *sab = reinterpret_cast<double *>(cur);  // a[64], b[64]
-  float2 *red_a = reinterpret_cast<float2 *>(sab + 128);  // per-warp double-float partials
+  float2 *sum_a = reinterpret_cast<float2 *>(cur);  // <P,HP> and |w|^2 of every step, double-floats
+  float2 *sum_b = sum_a + 64;
+  float2 *red_a = sum_b + 64;  // per-warp double-float partials
   float2 *red_b = red_a + kMaxWarps;
-  cur += sizeof(double) * (2 * kMaxWarps + 128);
+  cur += sizeof(float2) * (2 * kMaxWarps + 128);
   // gathered c per (warp, image): warp w's range covers images k_first(w).. so k + w is
   // unique for every pair it visits; plain stores, summed per slot in a fixed order
   float *part = reinterpret_cast<float *>(cur);
@@ -292,20 +356,22 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
   int *koff = kept + maxi;      // maxi + 1
   int *slot_first = koff + maxi + 1;  // first image of every slot (images sorted by atom)
   int *cnt = slot_first + maxi;  // [0] images, [1] slots, [2] overflow, [3] next node
-  // Veff rings of pass A (p.vring): slot s of thread t at s * kVRingThreads + t, so a warp's
-  // accesses to one slot are 512 contiguous bytes (no bank conflicts); 16-byte aligned
-  float4 *vring = reinterpret_cast<float4 *>(
-      (reinterpret_cast<uintptr_t>(cnt + 4) + 15) & ~static_cast<uintptr_t>(15));
 
   typename Rec::vec_t *rec = reinterpret_cast<typename Rec::vec_t *>(
       proj_scratch + (size_t)blockIdx.x * p.proj_bytes_per_cta);
   unsigned *ridx = reinterpret_cast<unsigned *>(
       reinterpret_cast<unsigned char *>(rec) + (size_t)p.proj_cap * sizeof(typename Rec::vec_t) * Rec::nvec);
 
-  const float4 *P4c = reinterpret_cast<const float4 *>(P);
   float4 *P4 = reinterpret_cast<float4 *>(P);
   float4 *U4 = reinterpret_cast<float4 *>(U);
   const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  // byte addresses: P, U, a quad of zeros that stands for every plane and row outside the cube
+  const unsigned sP = smem_addr(P), sU = smem_addr(U);
+  float4 *zq = reinterpret_cast<float4 *>(
+      (reinterpret_cast<uintptr_t>(cnt + 4) + 15) & ~static_cast<uintptr_t>(15));
+  const unsigned sZ = smem_addr(zq);
+  if (threadIdx.x == 0) *zq = zero4;  // the node loop's first barrier comes before its first use
+  const int PB = 16 * PS4, RB = 16 * nq;  // bytes of a plane and of a row
   const unsigned long long kpol = l2_keep_policy();
   static_assert(std::is_same<typename Rec::vec_t, float4>::value, "FP32 records of float4");
 
@@ -326,6 +392,7 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
   // x neighbours of the quad inside the row; lanes of the last quad zero its pad points
   const bool hm1 = ql >= 1, hm2 = ql >= 2, hp1 = ql + 1 < nq, hp2 = ql + 2 < nq;
   const int x0 = 4 * ql;
+  const int row4 = yA * nq + ql;  // pass A: quad index of (x0, yA) in a plane
   const bool in1 = x0 + 1 < nx, in2 = x0 + 2 < nx, in3 = x0 + 3 < nx;  // x0 < nx always
 
   // nodes: the first round one per CTA, then a queue (status[1], zeroed before the launch):
@@ -521,10 +588,12 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
     const size_t VPS4 = (size_t)p.EY * (p.vq_row >> 2);  // plane stride in quads
     const size_t VRS4 = (size_t)(p.vq_row >> 2);         // row stride in quads
 
-    float tb = 1.f;  // b_{k-1}
+    float sc = 1.f;          // s_k
+    DF n2 = {1.f, 0.f};      // |P|^2
+    DF gam = {0.f, 0.f};     // gamma_k
+    int steps = 0;
     for (int j = 0; j < p.nqp; j++) {
-      const float inv = 1.f / tb;
-      const float2 inv2 = splat(inv), ntb2 = splat(-tb);
+      const float2 sc2 = splat(sc), ngh2 = splat(-gam.hi), ngl2 = splat(-gam.lo);
 
       // ---- phase 1: projector gather  ||  pass A ----
       {
@@ -562,84 +631,62 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
       }
       Kahan ka;
       if (actA) {
-        // stencil weights scaled by 1/b_{k-1} (live in registers during this pass only)
         float2 czs[O + 1], cxs[O + 1];
 #pragma unroll
         for (int d = 1; d <= O; d++) {
-          czs[d] = splat(p.czf[d] * inv);
-          cxs[d] = ISO ? czs[d] : splat(p.cxf[d] * inv);
+          czs[d] = splat(p.czf[d]);
+          cxs[d] = ISO ? czs[d] : splat(p.cxf[d]);
         }
-        const int row4 = yA * nq + ql;  // quad index of (x0, yA) in a plane
-        const float4 *vrow = vq + (size_t)(K * p.EY + J + yA) * VRS4 + ql;
+        const float4 *vrow = vq + (size_t)(K * p.EY + J + yA) * VRS4 + ql + (size_t)zbA * VPS4;
+        // the quad at plane zbA + i of P and U, and P's plane 6 further on: all lanes make zlen
+        // steps (a uniform loop), those past their range keep nothing
+        unsigned aP = sP + 16u * (unsigned)(row4 + zbA * PS4 + pofs4);
+        unsigned aN = aP + (unsigned)(O * PB);
+        unsigned aU = sU + 16u * (unsigned)(row4 + zbA * PS4 + uofs4);
+        const int live = zeA - zbA, above = nz - O - zbA;
         float4 ring[W];
 #pragma unroll
         for (int q = -O; q < O; q++) {
           const int zq = zbA + q;
-          ring[q + O + 1] = (zq >= 0 && zq < nz) ? P4c[row4 + zq * PS4 + pofs4] : zero4;
+          ring[q + O + 1] = lds_quad(zq >= 0 && zq < nz ? aP + (unsigned)(q * PB) : sZ);
         }
         // x neighbours: the upper half of quad q-2, quads q-1 and q+1, the lower half of q+2
         float2 xm2 = make_float2(0.f, 0.f), xp2 = make_float2(0.f, 0.f);
         float4 xm1 = zero4, xp1 = zero4;
-        const float2 *P2c = reinterpret_cast<const float2 *>(P);
-        // U of plane z+1 loads while plane z is computed, and Veff (from L2) kVRingSlots - 1
-        // planes ahead through the thread's ring of async copies (p.vring; else one plane
-        // ahead in registers).  The 16-warp budget has no registers to spare for either.
-        constexpr bool kPrefetch = MAXT <= 384;
-        constexpr int kAhead = kVRingSlots - 1;
-        const bool use_ring = kPrefetch && p.vring;
-        const unsigned vr0 = (unsigned)__cvta_generic_to_shared(vring + threadIdx.x);
-        auto vcopy = [&](int zc, int slot) {  // Veff quad of plane zc into ring slot
-          if (zc < zeA)
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(
-                             vr0 + 16u * (unsigned)(slot * kVRingThreads)),
-                         "l"(__cvta_generic_to_global(vrow + (size_t)zc * VPS4))
-                         : "memory");
-          asm volatile("cp.async.commit_group;" ::: "memory");  // one group per plane, even empty
-        };
-        float4 nuo = zero4, ndv = zero4;
-        if constexpr (kPrefetch) {
-          nuo = U4[row4 + zbA * PS4 + uofs4];
-          if (use_ring) {
-            for (int d = 0; d < kAhead; d++) vcopy(zbA + d, d);
-          } else {
-            ndv = __ldg(vrow + (size_t)zbA * VPS4);
-          }
+        // U one plane ahead, Veff (from L2) two; the 16-warp budget has no registers for either
+        constexpr bool kAhead = MAXT <= 384;
+        float4 nuo = zero4, dv1 = zero4, dv2 = zero4;
+        if constexpr (kAhead) {
+          nuo = lds_quad(aU);
+          dv1 = __ldg(vrow);
+          dv2 = ldg_quad_if(1 < live, vrow + VPS4);
+          vrow += 2 * VPS4;
         }
-        for (int z0 = zbA; z0 < zeA; z0 += W) {
+        for (int i0 = 0; i0 < zlen; i0 += W) {
 #pragma unroll
           for (int s = 0; s < W; s++) {
-            const int z = z0 + s;
-            if (z >= zeA) break;
-            const int qn = z + O;
-            ring[s] = qn < nz ? P4c[row4 + qn * PS4 + pofs4] : zero4;
+            const int i = i0 + s;
+            if (i >= zlen) break;
+            ring[s] = lds_quad(i < above ? aN : sZ);
 #define RING(dd) ring[(s + (dd) + O + 1) % W]
-            const int i4 = row4 + z * PS4 + pofs4, iu4 = row4 + z * PS4 + uofs4;
-            if (hm2) xm2 = P2c[2 * i4 - 3];
-            if (hm1) xm1 = P4c[i4 - 1];
-            if (hp1) xp1 = P4c[i4 + 1];
-            if (hp2) xp2 = P2c[2 * i4 + 4];
+            lds_pair_if(hm2, aP - 24u, xm2);
+            lds_quad_if(hm1, aP - 16u, xm1);
+            lds_quad_if(hp1, aP + 16u, xp1);
+            lds_pair_if(hp2, aP + 32u, xp2);
             const float4 c = RING(0);
             float4 dv, uo;
-            if constexpr (kPrefetch) {
-              if (use_ring) {
-                // plane z's copy is done once at most kAhead - 1 later groups are pending; the
-                // copy of plane z + kAhead then goes to the slot read one plane earlier
-                asm volatile("cp.async.wait_group %0;" ::"n"(kAhead - 1) : "memory");
-                const int i = z - zbA;
-                dv = vring[(i & (kVRingSlots - 1)) * kVRingThreads + threadIdx.x];
-                vcopy(z + kAhead, (i + kAhead) & (kVRingSlots - 1));
-              } else {
-                dv = ndv;
-                if (z + 1 < zeA) ndv = __ldg(vrow + (size_t)(z + 1) * VPS4);
-              }
+            if constexpr (kAhead) {
+              dv = dv1;
+              dv1 = dv2;
+              dv2 = ldg_quad_if(i + 2 < live, vrow);
               uo = nuo;
-              if (z + 1 < zeA) nuo = U4[iu4 + PS4];
+              lds_quad_if(i + 1 < live, aU + (unsigned)PB, nuo);
             } else {
-              dv = __ldg(vrow + (size_t)z * VPS4);
-              uo = U4[iu4];
+              dv = ldg_quad_if(i < live, vrow);
+              uo = lds_quad(i < live ? aU : sZ);
             }
-            const float2 vs01 = mul2(lo(c), inv2), vs23 = mul2(hi(c), inv2);  // v_k
-            float2 h01 = mul2(lo(dv), vs01), h23 = mul2(hi(dv), vs23);
+            vrow += VPS4;
+            float2 h01 = mul2(lo(dv), lo(c)), h23 = mul2(hi(dv), hi(c));
 #pragma unroll
             for (int d = 1; d <= O; d++) {
               h01 = fma2(czs[d], add2(lo(RING(-d)), lo(RING(d))), h01);
@@ -659,61 +706,70 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
                 h23 = fma2(cxs[d], make_float2(e[8 - d] + e[8 + d], e[9 - d] + e[9 + d]), h23);
               }
             }
-            // zero the pad points, U <- h - b_{k-1} U, a_k partial <v_k, h>
+            // zero the pad points; U <- s h - gamma U; a_k partial <P, h>
             h01.y = in1 ? h01.y : 0.f;
             h23.x = in2 ? h23.x : 0.f;
             h23.y = in3 ? h23.y : 0.f;
-            const float2 n01 = fma2(ntb2, lo(uo), h01), n23 = fma2(ntb2, hi(uo), h23);
-            U4[iu4] = make_float4(n01.x, n01.y, n23.x, n23.y);
-            const float2 pa = fma2(vs01, h01, mul2(vs23, h23));
-            ka.add(pa.x + pa.y);
+            const float2 n01 = fma2(sc2, h01, fma2(ngh2, lo(uo), mul2(ngl2, lo(uo))));
+            const float2 n23 = fma2(sc2, h23, fma2(ngh2, hi(uo), mul2(ngl2, hi(uo))));
+            sts_quad_if(i < live, aU, make_float4(n01.x, n01.y, n23.x, n23.y));
+            const float2 pa = fma2(lo(c), h01, mul2(hi(c), h23));
+            ka.add(i < live ? pa.x + pa.y : 0.f);
+            aP += (unsigned)PB;
+            aN += (unsigned)PB;
+            aU += (unsigned)PB;
           }
         }
       }
       __syncthreads();
 
-      // ---- phase 2: pass B  ||  alpha = Gamma c / b ----
+      // ---- phase 2: pass B  ||  alpha = Gamma s c ----
       if (actB) {
         float2 cys[O + 1];
 #pragma unroll
-        for (int d = 1; d <= O; d++) cys[d] = splat((ISO ? p.czf[d] : p.cyf[d]) * inv);
-        // quad index of (x0, y = 0) in plane zB of P and of U
-        const int pl4 = zB * PS4 + ql + pofs4, pl4u = zB * PS4 + ql + uofs4;
+        for (int d = 1; d <= O; d++) cys[d] = splat(ISO ? p.czf[d] : p.cyf[d]);
+        // the quad at row ybB + i of P and U, and P's row 7 further on; all lanes make ylen steps
+        unsigned aP = sP + 16u * (unsigned)(zB * PS4 + ql + pofs4 + ybB * nq);
+        unsigned aN = aP + (unsigned)((O + 1) * RB);
+        unsigned aU = sU + 16u * (unsigned)(zB * PS4 + ql + uofs4 + ybB * nq);
+        const int live = yeB - ybB, above = ny - (O + 1) - ybB;
         // ring[j] holds row ybB - 6 + j; row y+7 and U of row y+1 load while row y computes
         float4 ring[W];
 #pragma unroll
         for (int j = 0; j < W; j++) {
           const int yq = ybB - O + j;
-          ring[j] = (yq >= 0 && yq < ny) ? P4c[pl4 + yq * nq] : zero4;
+          ring[j] = lds_quad(yq >= 0 && yq < ny ? aP + (unsigned)((j - O) * RB) : sZ);
         }
-        float4 nuo = U4[pl4u + ybB * nq];
-        for (int y0 = ybB; y0 < yeB; y0 += W) {
+        float4 nuo = lds_quad(aU);
+        for (int i0 = 0; i0 < ylen; i0 += W) {
 #pragma unroll
           for (int s = 0; s < W; s++) {
-            const int y = y0 + s;
-            if (y >= yeB) break;
-            const int u4 = pl4 + y * nq, uu4 = pl4u + y * nq;
+            const int i = i0 + s;
+            if (i >= ylen) break;
             const float4 uo = nuo;
-            const float4 nring = y + O + 1 < ny ? P4c[u4 + (O + 1) * nq] : zero4;
-            if (y + 1 < yeB) nuo = U4[uu4 + nq];
+            const float4 nring = lds_quad(i < above ? aN : sZ);
+            lds_quad_if(i + 1 < live, aU + (unsigned)RB, nuo);
 #define RING(dd) ring[(s + (dd) + O) % W]
-            float2 h01 = make_float2(0.f, 0.f), h23 = make_float2(0.f, 0.f);
+            float2 h01 = mul2(cys[1], add2(lo(RING(-1)), lo(RING(1))));
+            float2 h23 = mul2(cys[1], add2(hi(RING(-1)), hi(RING(1))));
 #pragma unroll
-            for (int d = 1; d <= O; d++) {
+            for (int d = 2; d <= O; d++) {
               h01 = fma2(cys[d], add2(lo(RING(-d)), lo(RING(d))), h01);
               h23 = fma2(cys[d], add2(hi(RING(-d)), hi(RING(d))), h23);
             }
             const float4 c = RING(0);
 #undef RING
-            const float2 n01 = add2(lo(uo), h01), n23 = add2(hi(uo), h23);
-            U4[uu4] = make_float4(n01.x, n01.y, n23.x, n23.y);
-            const float2 pa = fma2(mul2(lo(c), inv2), h01, mul2(mul2(hi(c), inv2), h23));
-            ka.add(pa.x + pa.y);
+            const float2 n01 = fma2(sc2, h01, lo(uo)), n23 = fma2(sc2, h23, hi(uo));
+            sts_quad_if(i < live, aU, make_float4(n01.x, n01.y, n23.x, n23.y));
+            const float2 pa = fma2(lo(c), h01, mul2(hi(c), h23));
+            ka.add(i < live ? pa.x + pa.y : 0.f);
             ring[s] = nring;  // row y-6 leaves, row y+7 joins
+            aN += (unsigned)RB;
+            aU += (unsigned)RB;
           }
         }
       }
-      // alpha = Gamma_l c, with c = <chi, v_k>; <v_k, V_nl v_k> = sum Gamma_l c^2 joins a_k
+      // alpha = Gamma_l s c, with c = <chi, P>; <P, V_nl P> = sum Gamma_l c^2 joins the a_k sum
       for (int e = threadIdx.x; e < n_slot * NLM; e += blockDim.x) {
         const int sl = e / NLM, r = e - sl * NLM;
         const TypeDesc &td = p.types[slot_type[sl]];
@@ -730,11 +786,10 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
           cx[cr * maxi * NLM + e] = csum;
           *cooperative_groups::this_cluster().map_shared_rank(cx + cr * maxi * NLM + e, cr ^ 1) = csum;
         } else {
-          const float cv = csum * inv;
           const float gl = (td.chan_mask & (1 << l)) ? float(td.gamma[l]) : 0.f;
-          const float al = gl * cv;
-          alpha[e] = al;
-          ka.add(al * cv);
+          const float al = gl * csum;
+          alpha[e] = al * sc;
+          ka.add(al * csum);
         }
       }
       {
@@ -751,14 +806,14 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
           const int kend = min(r_end, koff[k + 1]);
           const int shift = pref[k] - koff[k];
           float coef[NLM];
-          if constexpr (PAIR) {  // alpha = Gamma_l (c_0 + c_1) / b from the two CTAs' rows
+          if constexpr (PAIR) {  // alpha = Gamma_l s (c_0 + c_1) from the two CTAs' rows
             const int sl = slot[k];
             const TypeDesc &td = p.types[slot_type[sl]];
 #pragma unroll
             for (int s = 0; s < NLM; s++) {
               const int l = p.rank_l[s];
               const float gl = (td.chan_mask & (1 << l)) ? float(td.gamma[l]) : 0.f;
-              coef[s] = gl * ((cx[sl * NLM + s] + cx[maxi * NLM + sl * NLM + s]) * inv);
+              coef[s] = gl * ((cx[sl * NLM + s] + cx[maxi * NLM + sl * NLM + s]) * sc);
             }
           } else {
             const float *al = alpha + slot[k] * NLM;
@@ -789,14 +844,14 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
       }
       DF adf;
       if constexpr (PAIR) {
-        // <v, V_nl v> = sum Gamma_l c^2 over the slots, the same sum in both CTAs
+        // <P, V_nl P> = sum Gamma_l c^2 over the slots, the same sum in both CTAs
         Kahan kn;
         for (int e = threadIdx.x; e < n_slot * NLM; e += blockDim.x) {
           const int sl = e / NLM, r = e - sl * NLM;
           const TypeDesc &td = p.types[slot_type[sl]];
           const int l = p.rank_l[r];
           const float gl = (td.chan_mask & (1 << l)) ? float(td.gamma[l]) : 0.f;
-          const float cv = (cx[e] + cx[maxi * NLM + e]) * inv;
+          const float cv = cx[e] + cx[maxi * NLM + e];
           kn.add(gl * cv * cv);
         }
         const DF np = df_warp_sum(df_of(kn));
@@ -814,7 +869,8 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
 
       // ---- phase 4: w = U - a_k v, P <- w, U <- v, b_k^2 partial ----
       {
-        const float2 na2 = splat(-(adf.hi + adf.lo));
+        const DF ak = df_div(adf, n2);
+        const float2 nah2 = splat(-ak.hi), nal2 = splat(-ak.lo);
         Kahan kb;
         // owned planes: P's at quad e + udelta/4, U's at e.  PAIR: quads [h0, h1) are the
         // peer's halo planes and also go to its P at e + dpeer.
@@ -841,8 +897,9 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
             npv = P4o[e + blockDim.x];
             nuv = U4[e + blockDim.x];
           }
-          const float2 v01 = mul2(lo(pv), inv2), v23 = mul2(hi(pv), inv2);
-          const float2 w01 = fma2(na2, v01, lo(uv)), w23 = fma2(na2, v23, hi(uv));
+          const float2 v01 = mul2(lo(pv), sc2), v23 = mul2(hi(pv), sc2);
+          const float2 w01 = fma2(nal2, v01, fma2(nah2, v01, lo(uv)));
+          const float2 w23 = fma2(nal2, v23, fma2(nah2, v23, hi(uv)));
           const float4 w4 = make_float4(w01.x, w01.y, w23.x, w23.y);
           P4o[e] = w4;
           if constexpr (PAIR) {
@@ -854,7 +911,7 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
         }
         const DF bp = df_warp_sum(df_of(kb));
         if (lane == 0) red_b[warp] = make_float2(bp.hi, bp.lo);
-        if (threadIdx.x == 0) sab[j] = (double)adf.hi + (double)adf.lo;
+        if (threadIdx.x == 0) sum_a[j] = make_float2(adf.hi, adf.lo);
       }
       DF b2;
       if constexpr (PAIR) {  // the halo planes and both CTAs' b partials are in place
@@ -867,26 +924,34 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
         __syncthreads();
         b2 = df_all_reduce(red_b, nw);
       }
-      const float bf = sqrtf(b2.hi + b2.lo);
-      if (threadIdx.x == 0) sab[64 + j] = sqrt((double)b2.hi + (double)b2.lo);
-      if (!(bf > 0.f) || !isfinite(bf)) {  // breakdown: the Krylov space is invariant
-        if (threadIdx.x == 0) {
-          atomicOr(status, kStatusBreakdown);
-          for (int r = j + 1; r < p.nqp; r++) {
-            sab[r] = 0.0;
-            sab[64 + r] = 0.0;
-          }
-        }
+      if (threadIdx.x == 0) sum_b[j] = make_float2(b2.hi, b2.lo);
+      steps = j + 1;
+      if (!(b2.hi > 0.f) || !isfinite(b2.hi)) {  // breakdown: the Krylov space is invariant
+        if (threadIdx.x == 0) atomicOr(status, kStatusBreakdown);
         break;
       }
-      tb = bf;
+      // the next vector's scale, the power of two that brings |s P|^2 into [1, 4), and
+      // gamma = <s' w, H s P> / |s P|^2 = s' |w|^2 / (s^2 |P|^2)
+      const float nsc = unit_scale(b2.hi);
+      const DF g = df_div(b2, n2);
+      const float gs = nsc / (sc * sc);
+      gam = DF{g.hi * gs, g.lo * gs};
+      n2 = b2;
+      sc = nsc;
     }
     __syncthreads();
     if (cr == 0)
       for (int r = threadIdx.x; r < p.nqp; r += blockDim.x) {
+        double av = 0.0, bv = 0.0;  // after a breakdown
+        if (r < steps) {
+          const float2 one = make_float2(1.f, 0.f), np = r ? sum_b[r - 1] : one;
+          const double n = (double)np.x + np.y;
+          av = ((double)sum_a[r].x + sum_a[r].y) / n;
+          bv = sqrt(((double)sum_b[r].x + sum_b[r].y) / n) / (double)(r ? unit_scale(np.x) : 1.f);
+        }
         double *o = ab_out + (node - p.node_begin) * 2 * p.nqp;
-        o[r] = sab[r];
-        o[p.nqp + r] = sab[64 + r];
+        o[r] = av;
+        o[p.nqp + r] = bv;
       }
     __syncthreads();
   }
