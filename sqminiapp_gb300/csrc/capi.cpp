@@ -117,10 +117,11 @@ int max_images_per_node(const sq::Setup &s, const sq::Deck &d) {
   return best;
 }
 
-// Largest number of (image, box point) pairs inside one node's cube.  The overlap of an image
-// box with the cube of node (I,J,K) is a product of three 1D overlaps, so every image adds
-// ov_x(I) ov_y(J) ov_z(K) over the nodes whose cubes it meets.
-long long max_box_points_per_node(const sq::Setup &s, const sq::Deck &d) {
+// Largest sum over images, at any node, of a count that is a product of three 1D counts:
+// count(axis, lo, hi) for an image box that covers the cube's points [lo, hi] of that axis (cube
+// coordinates).
+template <typename F>
+long long max_image_sum_per_node(const sq::Setup &s, const sq::Deck &d, F &&count) {
   const int N[3] = {d.grid[0], d.grid[1], d.grid[2]};
   std::vector<long long> acc((size_t)N[0] * N[1] * N[2], 0);
   for (const sq::ImageMeta &im : s.images) {
@@ -134,7 +135,8 @@ long long max_box_points_per_node(const sq::Setup &s, const sq::Deck &d) {
       const int hi = std::min(N[a] - 1, b[a] + f[a] - 1 + s.nh[a]);
       if (hi < lo[a]) empty = true;
       for (int I = lo[a]; I <= hi; I++)
-        ov[a].push_back(std::min(b[a] + f[a] - 1, I + s.nh[a]) - std::max(b[a], I - s.nh[a]) + 1);
+        ov[a].push_back(count(a, std::max(b[a], I - s.nh[a]) - (I - s.nh[a]),
+                              std::min(b[a] + f[a] - 1, I + s.nh[a]) - (I - s.nh[a])));
     }
     if (empty) continue;
     for (size_t kz = 0; kz < ov[2].size(); kz++)
@@ -147,6 +149,41 @@ long long max_box_points_per_node(const sq::Setup &s, const sq::Deck &d) {
   long long best = 0;
   for (long long v : acc) best = std::max(best, v);
   return best;
+}
+
+// (image, box point) pairs inside one node's cube.
+long long max_box_points_per_node(const sq::Setup &s, const sq::Deck &d) {
+  return max_image_sum_per_node(s, d, [](int, int lo, int hi) { return hi - lo + 1; });
+}
+
+// Bounds of the split-pass kernel's projector list with `block` threads per CTA: units of a node
+// (every column of quads of every image's box, cut at the items' plane ranges) and batches of 32
+// (the items are dealt out in the order of their units, so a warp's lanes differ by little).
+// False if the unit words cannot hold them.
+bool quad_list_bounds(const sq::Setup &s, const sq::Deck &d, sq::LanczosParams &p, int block) {
+  const int columns = (p.pitch / 4) * p.ny;
+  const int ends[3] = {0, (p.layout & sq::kLayoutPair) ? p.zsplit : p.nz, p.nz};
+  long long units = 0;
+  int most = 0;
+  for (int r = 0; r < 2; r++) {
+    const int z0 = ends[r], planes = ends[r + 1] - ends[r];
+    if (planes == 0) continue;
+    const int chunks = sq::lanczos_quad_list_chunks(columns, planes, block);
+    units = std::max(units, max_image_sum_per_node(s, d, [&](int a, int lo, int hi) {
+      if (a == 0) return (hi >> 2) - (lo >> 2) + 1;
+      if (a == 1) return hi - lo + 1;
+      int n = 0;
+      for (int c = 0; c < chunks; c++) {
+        const int b0 = z0 + planes * c / chunks, b1 = z0 + planes * (c + 1) / chunks;
+        n += (std::max(0, std::min(hi + 1, b1) - std::max(lo, b0)) + sq::kQuadListRun - 1) / sq::kQuadListRun;
+      }
+      return n;
+    }));
+    most = std::max(most, p.max_img * (((planes + chunks - 1) / chunks + sq::kQuadListRun - 1) / sq::kQuadListRun));
+  }
+  p.part_total = std::max(p.part_total, (int)std::min<long long>(units, 1 << 20));
+  p.list_batches = std::max<int>(p.list_batches, p.part_total / 32 + 2 * most + block / 32 + 2);
+  return p.part_total < 65536 && p.max_img < 1024;
 }
 
 // Mean over all nodes of sum_images |box ∩ cube|.  The overlap of a box with the cube of
@@ -310,29 +347,43 @@ void plan_engine(sq_handle *h, int smem_optin, int l2_bytes) {
   p.zchunks = 1;
   p.ychunks = 1;
   p.zsplit = 0;
+  p.proj_cap = p.part_total = p.list_batches = p.part_cap = 0;
   p.vq_row = 4 * ((p.EX + 6 + 3) / 4);  // the row of a quad-aligned Veff copy (see below)
   p.vq_copy_stride = (long long)p.vq_row * p.EY * p.EZ;
   h->quad = false;
   if (h->opt.kernel < 0 || h->opt.kernel > 2 || h->opt.tile < 0)
     throw std::invalid_argument("sq_options.kernel must be 0, 1 or 2 and tile >= 0");
   if (h->opt.precision == 32 && !faithful && h->opt.kernel != 1 && h->opt.list_format != 2) {
-    // split-pass kernel over 16-byte quads: P and U on chip as [nz][ny][4 ceil(nx/4)], full
-    // projector records, which must stay in L2 together (152 CTAs' lists)
+    // split-pass kernel over 16-byte quads: P and U on chip as [nz][ny][4 ceil(nx/4)], the
+    // projector list in tensor memory
     sq::LanczosParams q = p;
     q.layout = sq::kLayoutQuad;
     q.pitch = q.upitch = 4 * ((p.nx + 3) / 4);
     q.zchunks = h->opt.tile > 0 ? h->opt.tile : 2;
     const int threads = sq::lanczos_quad_threads(q);
-    const double list_bytes = (double)h->num_sms * projector_points_per_node(s, d) *
-                              kept_fraction(s) *
-                              (double)sq::proj_record_bytes(4, false, p.union_mask, false);
-    if (!wide && threads <= sq::kQuadMaxThreads &&
+    // list bounds for every tile that may run
+    q.part_total = q.list_batches = q.part_cap = 0;
+    bool words = true;
+    for (int tile = h->opt.tile > 0 ? h->opt.tile : 1; tile <= std::max(4, h->opt.tile); tile++) {
+      sq::LanczosParams t = q;
+      t.zchunks = tile;
+      if (wide || sq::lanczos_quad_threads(t) > sq::kQuadMaxThreads) break;
+      words = quad_list_bounds(s, d, q, sq::lanczos_quad_block(t)) && words;
+      if (h->opt.tile > 0) break;
+    }
+    // The lists of all CTAs, were none of them in tensor memory, must stay in L2 (what exceeds it is
+    // streamed from there): units of whole boxes, about half of which the spheres fill.
+    auto list_bytes = [&](const sq::LanczosParams &l) {
+      return (double)h->num_sms * 0.6 * l.part_total * (double)sq::lanczos_quad_unit_bytes(l);
+    };
+    if (!wide && threads <= sq::kQuadMaxThreads && words &&
         sq::lanczos_quad_smem_bytes(q) <= (size_t)smem_optin &&
-        (h->opt.list_format == 1 || list_bytes <= 0.75 * (double)l2_bytes)) {
+        (h->opt.list_format == 1 || list_bytes(q) <= 0.75 * (double)l2_bytes)) {
       p = q;
       h->quad = true;
       h->u_smem = true;
       h->block = sq::lanczos_quad_block(q);
+      sq::lanczos_quad_place_partials(p, smem_optin);
     } else if (h->opt.tile == 0 && p.nz >= 2 * sq::kStencilHalf + 2) {
       // the same kernel on a pair of CTAs per node, the cube split in z: each holds its half
       // of U and its half of P plus 6 halo planes; each streams its half of the list
@@ -340,19 +391,22 @@ void plan_engine(sq_handle *h, int smem_optin, int l2_bytes) {
       q.zsplit = (p.nz + 1) / 2;
       q.zchunks = 1;
       q.ychunks = 2;
+      q.part_total = q.list_batches = 0;
+      words = quad_list_bounds(s, d, q, sq::kPairThreads);
       int pt = sq::lanczos_quad_threads(q);
       if (pt > sq::kPairThreads) {
         q.ychunks = 1;
         pt = sq::lanczos_quad_threads(q);
       }
-      if (pt <= sq::kPairThreads && sq::lanczos_quad_smem_bytes(q) <= (size_t)smem_optin &&
-          (h->opt.list_format == 1 || 0.5 * list_bytes <= 0.75 * (double)l2_bytes)) {
+      if (pt <= sq::kPairThreads && words && sq::lanczos_quad_smem_bytes(q) <= (size_t)smem_optin &&
+          (h->opt.list_format == 1 || list_bytes(q) <= 0.75 * (double)l2_bytes)) {
         p = q;
         h->quad = true;
         h->u_smem = true;
         // all 12 warps of the register budget: the stencil passes use pt threads, the list
         // streams and the update all of them (fewer, longer warp ranges are slower)
         h->block = sq::kPairThreads;
+        sq::lanczos_quad_place_partials(p, smem_optin);
         h->tuned = true;  // one tile
       }
     }
@@ -412,13 +466,17 @@ void plan_engine(sq_handle *h, int smem_optin, int l2_bytes) {
     if (psize >= 65536 || (long long)p.upitch * p.ny * p.nz >= 65536)
       throw std::invalid_argument("truncated cube too large for 16-bit point indices");
   }
-  const long long cap = std::max(1LL, max_box_points_per_node(s, d));
-  if (cap > (1LL << 31) - 1) throw std::invalid_argument("projector list too large");
-  p.proj_cap = (int)cap;
-  p.proj_bytes_per_cta =
-      (long long)((cap * sq::proj_record_bytes((int)h->elem, faithful, p.union_mask,
-                                               (p.layout & sq::kLayoutCompact) != 0) +
-                   255) & ~255LL);
+  if (h->quad) {
+    p.proj_bytes_per_cta = (long long)((sq::lanczos_quad_list_bytes(p) + 255) & ~size_t(255));
+  } else {
+    const long long cap = std::max(1LL, max_box_points_per_node(s, d));
+    if (cap > (1LL << 31) - 1) throw std::invalid_argument("projector list too large");
+    p.proj_cap = (int)cap;
+    p.proj_bytes_per_cta =
+        (long long)((cap * sq::proj_record_bytes((int)h->elem, faithful, p.union_mask,
+                                                 (p.layout & sq::kLayoutCompact) != 0) +
+                     255) & ~255LL);
+  }
   fill_info(h->info, d, s, p.max_img, h->opt);
   h->info.kernel_layout = p.layout;
   h->info.kernel_u_on_chip = h->u_smem ? 1 : 0;

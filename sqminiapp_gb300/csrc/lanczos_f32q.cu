@@ -1,5 +1,7 @@
 // lanczos_f32q.cu -- instantiations of the split-pass FP32 Lanczos kernel (kLayoutQuad) and its
 // host-side sizes.
+#include <algorithm>
+
 #include "lanczos_quad.cuh"
 
 namespace sq {
@@ -26,17 +28,53 @@ size_t lanczos_quad_smem_bytes(const LanczosParams &p) {
   const bool pair = (p.layout & kLayoutPair) != 0;
   const size_t ps = lq::quad_plane_floats(p.ny, p.pitch);
   const int nlm = mask_nlm(kernel_mask(p.union_mask));
-  size_t b = pair ? sizeof(float) * ps * (lq::pair_p_planes(p.nz, p.zsplit) +
-                                          lq::pair_u_planes(p.nz, p.zsplit))
-                  : sizeof(float) * 2 * ps * p.nz;           // P, U
-  b += sizeof(double) * (2 * lk::kMaxWarps + 128);           // a_k / b_k partials, a[], b[]
-  b += sizeof(float) * (2 * (size_t)p.max_img + lk::kMaxWarps) * nlm;  // c partials, alpha
+  const size_t pu[2] = {  // planes of P and of U
+      (size_t)(pair ? lq::pair_p_planes(p.nz, p.zsplit) : lq::list_planes(p.nz)),
+      (size_t)(pair ? lq::pair_u_planes(p.nz, p.zsplit) : lq::list_planes(p.nz))};
+  size_t b = sizeof(float) * ps * (pu[0] + pu[1]);
+  b += sizeof(float2) * (2 * lk::kMaxWarps + 128);           // partials and step sums
+  b += sizeof(float) * (size_t)p.max_img * nlm;              // alpha
   if (pair)  // both CTAs' c, an 8-byte alignment, projector a_k partials, capacity flags
     b += sizeof(float) * 2 * (size_t)p.max_img * nlm + 8 + sizeof(float) * 2 * lk::kMaxWarps +
          sizeof(int) * 4;
-  b += sizeof(int) * (9 * (size_t)p.max_img + 2) + sizeof(int) * 4;    // per-node image lists
-  b += 16 + sizeof(float4);  // the quad of zeros
+  b += sizeof(int) * (4 * (size_t)p.max_img + 2 + 6 + lk::kMaxWarps);  // per-node lists
+  b += 16 + sizeof(lq::ImgRow) * (size_t)p.max_img + sizeof(float4);   // image rows, a quad of zeros
+  b += sizeof(float4) * (size_t)p.part_cap;
+  const size_t scratch = lq::list_scratch_bytes(p.max_img, kQuadMaxThreads / 32);
+  if (scratch > sizeof(float) * ps * pu[1]) b += scratch;  // list build, where U is too small for it
   return b;
+}
+
+static_assert(kQuadListRun == lq::kRun, "host and device agree on the list's units");
+int lanczos_quad_list_chunks(int columns, int planes, int threads) {
+  return lq::list_chunks(columns, planes, threads);
+}
+
+namespace {
+int channels(const LanczosParams &p) {
+  int n = 0;
+  for (int l = 0; l < 4; l++) n += (kernel_mask(p.union_mask) >> l) & 1;
+  return n;
+}
+size_t partial_float4(const LanczosParams &p) { return (mask_nlm(kernel_mask(p.union_mask)) + 3) / 4; }
+}  // namespace
+
+size_t lanczos_quad_unit_bytes(const LanczosParams &p) {
+  return sizeof(float4) * lq::kRun * channels(p) + sizeof(unsigned);
+}
+
+size_t lanczos_quad_list_bytes(const LanczosParams &p) {
+  return (size_t)p.list_batches * 32 * lanczos_quad_unit_bytes(p) +
+         sizeof(float4) * partial_float4(p) * (size_t)p.part_total;
+}
+
+void lanczos_quad_place_partials(LanczosParams &p, int smem_optin) {
+  // part_total counts whole boxes; the units of the spheres in them are about half (2161 of 4608 on
+  // a 27^3 cube).  A node with more keeps its partial sums in the scratch slice.
+  p.part_cap = 0;
+  const size_t room = ((size_t)smem_optin - lanczos_quad_smem_bytes(p)) / sizeof(float4);
+  const size_t want = partial_float4(p) * (size_t)(0.6 * p.part_total + 1);
+  p.part_cap = (int)std::min(room, want);
 }
 
 size_t veff_quad_floats(const LanczosParams &p) { return 4 * (size_t)p.vq_copy_stride; }

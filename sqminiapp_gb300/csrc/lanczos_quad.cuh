@@ -23,14 +23,21 @@
 // Eight consecutive threads own the quads of one row (pass A) or one plane (pass B), so a
 // quarter-warp's float4 accesses cover one contiguous row: no bank conflicts.
 //
-// Projector list: as in lanczos_kernel.cuh (chi_lm of the node's support points, built once
-// per node into the CTA's slice of global scratch), with one index per point (P and U share
-// it); consecutive lanes stream consecutive points, so every record load of a warp is one
-// contiguous 512-byte run.
+// Projector list.  Its unit is (image, column of quads, four planes): T_l of four quads above one
+// another (zero outside the support), and one word with the image, the first plane and the place of
+// the unit's partial sums; chi_lm = T_l P_lm(x,y,z) is formed while streaming, over a column with the
+// same x and y for every plane.  A thread owns one column over a range of planes and all its units
+// (dealt out by their number, so that the lanes of a warp have equally many): no two threads meet on a
+// quad, the scatter needs no atomics, and every run gives the same result.  The list is built once per
+// node and lives in the SM's tensor memory, which this kernel does not need for anything else
+// (tcgen05.ld: no L2 round trip, no shared memory); what exceeds its 512 columns goes to a slice of
+// global scratch.  The gather writes four (s+p) partial sums per unit, ordered by atom, to shared
+// memory where they fit, else to the scratch slice.
+//   Before, a list of points (20 bytes each) was streamed from L2 twice a step: 2 x 148 of 591
+// instructions per quad-warp and step, and the atomics of the scatter.
 //
 // Per Lanczos step (v_k = s_k P with s_k a power of two, U = v_{k-1}), four CTA barriers:
-//   1  projector gather c = chi^T P (per-warp ranges of the node's list, one partial per
-//      warp and image, no atomics)  ||  pass A
+//   1  projector gather c = chi^T P (partial sums per unit)  ||  pass A
 //   2  pass B  ||  alpha = Gamma s c (and <P, V_nl P>)  -> per-warp partials of <P, H P>
 //   3  projector scatter U += chi alpha  ||  every warp reduces the a_k partials
 //   4  w = U - a_k v, P <- w, U <- v  -> per-warp partials of b_k^2
@@ -50,8 +57,8 @@
 // most of the FP32 error (weights 6e-6 -> 4e-7 and the lowest Ritz value 5e-7 -> 5e-8 Ha on a 27^3
 // cube without projectors, the diagonal's share of the weights' rounding included).
 //
-// Memory traffic.  Pass A reads Veff from L2 two planes ahead.  The list's stores and loads carry
-// an L2 evict-last policy.  Nodes after the first round come from a device-side queue.
+// Memory traffic.  Pass A reads Veff from L2 two planes ahead.  Nodes after the first round come
+// from a device-side queue.
 //
 // CTA pair (PAIR, lanczos_quad_pair_kernel): one node per cluster of two CTAs for cubes whose
 // P and U do not fit one CTA.  The cube is split in z (PairPlanes); each CTA owns its planes of
@@ -64,6 +71,7 @@
 #include <cooperative_groups.h>
 
 #include "lanczos_kernel.cuh"
+#include "tc5.cuh"
 
 namespace sq {
 namespace lq {
@@ -229,58 +237,279 @@ __host__ __device__ constexpr int pair_u_planes(int nz, int zsplit) {
   return zsplit > nz - zsplit ? zsplit : nz - zsplit;
 }
 
-// The per-node projector list (records and point indices) is written once per node and read
-// twice per Lanczos step from L2: its stores and loads carry an L2 evict-last cache policy so
-// that other traffic does not push it out between the steps.
-__device__ __forceinline__ unsigned long long l2_keep_policy() {
-  unsigned long long pol;
-  asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
-  return pol;
+// ---- the projector list ----
+// A unit of the list is (image, column, kRun planes): the radial values T_l of kRun quads above one
+// another, zero outside the support and the run.  A thread owns one column of quads over a range of
+// planes ("item") and its units, so no two threads ever meet on a quad.
+constexpr int kRun = 4;
+constexpr int kListColumns = 512;                   // the whole tensor memory of an SM
+constexpr int kListHeads = 32;                      // columns of unit words; the rest holds T_l
+__host__ __device__ constexpr int list_units_per_quarter(int nch) {  // (a quarter: 32 of the 128 lanes)
+  return (kListColumns - kListHeads) / (4 * kRun * nch);
 }
-__device__ __forceinline__ void st_keep(float4 *p, float4 v, unsigned long long pol) {
-  asm volatile("st.global.L2::cache_hint.v4.f32 [%0], {%1, %2, %3, %4}, %5;" ::"l"(p), "f"(v.x),
-               "f"(v.y), "f"(v.z), "f"(v.w), "l"(pol)
-               : "memory");
+// Plane ranges per column: as many as the threads allow with at least kRun planes each.
+__host__ __device__ constexpr int list_chunks(int columns, int planes, int threads) {
+  int c = threads / columns < 1 ? 1 : threads / columns;
+  while (c > 1 && planes / c < kRun) c--;
+  return c;
 }
-__device__ __forceinline__ void st_keep(unsigned *p, unsigned v, unsigned long long pol) {
-  asm volatile("st.global.L2::cache_hint.u32 [%0], %1, %2;" ::"l"(p), "r"(v), "l"(pol) : "memory");
+__host__ __device__ constexpr int list_planes(int planes) {  // planes to allocate
+  return planes < kRun ? kRun : planes;
 }
-__device__ __forceinline__ float4 ld_keep(const float4 *p, unsigned long long pol) {
-  float4 v;
-  asm volatile("ld.global.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "l"(p), "l"(pol));
-  return v;
+constexpr int kSortKeys = 64;
+// Bytes of per-node scratch of the list build: a key histogram per warp, the items in order, unit
+// counts per (image, warp).
+__host__ __device__ constexpr int list_scratch_bytes(int max_img, int nw) {
+  return 4 * (kSortKeys * nw + 32 * nw + max_img * nw);
 }
-__device__ __forceinline__ unsigned ld_keep(const unsigned *p, unsigned long long pol) {
-  unsigned v;
-  asm volatile("ld.global.L2::cache_hint.u32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(pol));
-  return v;
+
+// Tensor memory: a warp reads and writes its own quarter of the lanes.
+__device__ __forceinline__ void tmem_ld16(unsigned taddr, float4 (&t)[4]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=f"(t[0].x), "=f"(t[0].y), "=f"(t[0].z), "=f"(t[0].w), "=f"(t[1].x), "=f"(t[1].y),
+        "=f"(t[1].z), "=f"(t[1].w), "=f"(t[2].x), "=f"(t[2].y), "=f"(t[2].z), "=f"(t[2].w),
+        "=f"(t[3].x), "=f"(t[3].y), "=f"(t[3].z), "=f"(t[3].w)
+      : "r"(taddr));
 }
-// one list record (N values of chi_lm, zero-padded to whole float4) with the policy above
-template <int N>
-__device__ __forceinline__ void rec_store_keep(float4 *rec, int e, const float *v,
-                                               unsigned long long pol) {
-  constexpr int nv = (N + 3) / 4;
+__device__ __forceinline__ void tmem_st16(unsigned taddr, const float4 (&t)[4]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};" ::"f"(
+          t[0].x),
+      "f"(t[0].y), "f"(t[0].z), "f"(t[0].w), "f"(t[1].x), "f"(t[1].y), "f"(t[1].z), "f"(t[1].w),
+      "f"(t[2].x), "f"(t[2].y), "f"(t[2].z), "f"(t[2].w), "f"(t[3].x), "f"(t[3].y), "f"(t[3].z),
+      "f"(t[3].w), "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld1(unsigned taddr, unsigned &a) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(a) : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_st1(unsigned taddr, unsigned a) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(taddr), "r"(a) : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() {
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+// The wait names the registers it guards, so that no use of them moves above it.
+template <int N> __device__ __forceinline__ void tmem_wait_ld(float4 (&t)[N][4], unsigned &w) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(w)::"memory");
 #pragma unroll
-  for (int j = 0; j < nv; j++) {
-    float t[4];
+  for (int c = 0; c < N; c++)
 #pragma unroll
-    for (int q = 0; q < 4; q++) t[q] = 4 * j + q < N ? v[4 * j + q] : 0.f;
-    st_keep(rec + (size_t)e * nv + j, make_float4(t[0], t[1], t[2], t[3]), pol);
+    for (int i = 0; i < 4; i++)
+      asm volatile("" : "+f"(t[c][i].x), "+f"(t[c][i].y), "+f"(t[c][i].z), "+f"(t[c][i].w));
+}
+
+// A unit's word: image (10 bits), first plane from the first owned one (6), place of its partial
+// sums (16).
+__device__ __forceinline__ unsigned unit_word(int image, int z0, int place) {
+  return (unsigned)(image | (z0 << 10)) | ((unsigned)place << 16);
+}
+// An image of the node: box point 0 in cube coordinates (z from the first owned plane) as floats,
+// its coordinates relative to the atom, type and atom slot.
+struct ImgRow {
+  float bx, by, bz, ox;
+  float oy, oz;
+  int type, slot;
+};
+static_assert(sizeof(ImgRow) == 32, "two 16-byte loads");
+__device__ __forceinline__ ImgRow load_row(const ImgRow *r) {
+  const float4 a = reinterpret_cast<const float4 *>(r)[0], b = reinterpret_cast<const float4 *>(r)[1];
+  return ImgRow{a.x, a.y, a.z, a.w, b.x, b.y, __float_as_int(b.z), __float_as_int(b.w)};
+}
+
+// Products of a unit's T with kRun quads of a column.  gather: the unit's raw sums (times norm() they
+// are <chi_lm, P>); scatter: adds sum_lm chi_lm q_lm, q with norm() in it.
+template <int MASK> struct UnitChi {
+  static constexpr int nch = (MASK & 1) + ((MASK >> 1) & 1) + ((MASK >> 2) & 1) + ((MASK >> 3) & 1);
+  static constexpr int nlm = lk::Lm<MASK>::nlm;
+  static __device__ __forceinline__ float norm(int) { return 1.f; }
+  // FN(channel, rank, harmonic) at (x, y, z)
+  template <typename FN>
+  static __device__ __forceinline__ void harmonics(float x, float y, float z, FN &&fn) {
+    int c = 0;
+    auto channel = [&](auto Lc) {
+      constexpr int L = decltype(Lc)::value;
+      if constexpr (MASK & (1 << L)) {
+        lk::solid_harmonics<L, float>(x, y, z, [&](int s, float ylm) { fn(c, lk::Lm<MASK>::rank(s), ylm); });
+        c++;
+      }
+    };
+    channel(std::integral_constant<int, 0>{});
+    channel(std::integral_constant<int, 1>{});
+    channel(std::integral_constant<int, 2>{});
+    channel(std::integral_constant<int, 3>{});
   }
+  static __device__ __forceinline__ float at(float4 v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
+  static __device__ __forceinline__ void gather(const LanczosParams &p, const float4 (&T)[nch][kRun],
+                                                const float4 (&v)[kRun], float x, float y, float z,
+                                                float (&c)[nlm]) {
+#pragma unroll
+    for (int s = 0; s < nlm; s++) c[s] = 0.f;
+#pragma unroll
+    for (int k = 0; k < kRun; k++)
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        float t[nch];
+#pragma unroll
+        for (int q = 0; q < nch; q++) t[q] = at(v[k], i) * at(T[q][k], i);
+        harmonics(fmaf(p.hxf, float(i), x), y, fmaf(p.hzf, float(k), z),
+                  [&](int q, int r, float ylm) { c[r] = fmaf(ylm, t[q], c[r]); });
+      }
+  }
+  static __device__ __forceinline__ void scatter(const LanczosParams &p, const float4 (&T)[nch][kRun],
+                                                 float4 (&u)[kRun], float x, float y, float z,
+                                                 const float (&q)[nlm]) {
+#pragma unroll
+    for (int k = 0; k < kRun; k++) {
+      float r4[4] = {u[k].x, u[k].y, u[k].z, u[k].w};
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        float g[nch];
+#pragma unroll
+        for (int c = 0; c < nch; c++) g[c] = 0.f;
+        harmonics(fmaf(p.hxf, float(i), x), y, fmaf(p.hzf, float(k), z),
+                  [&](int c, int r, float ylm) { g[c] = fmaf(ylm, q[r], g[c]); });
+#pragma unroll
+        for (int c = 0; c < nch; c++) r4[i] = fmaf(at(T[c][k], i), g[c], r4[i]);
+      }
+      u[k] = make_float4(r4[0], r4[1], r4[2], r4[3]);
+    }
+  }
+};
+// s and p channels, two points per instruction: over a column x and y are the same for every plane,
+// so their sums are taken once per unit.  Ranks: s, y, z, x.
+template <> struct UnitChi<3> {
+  static constexpr int nch = 2, nlm = 4;
+  static __device__ __forceinline__ float norm(int r) { return r == 0 ? 1.f : 0.488602511902920f; }
+  static __device__ __forceinline__ void gather(const LanczosParams &p, const float4 (&T)[nch][kRun],
+                                                const float4 (&v)[kRun], float x, float y, float z,
+                                                float (&c)[nlm]) {
+    float2 s = mul2(lo(T[0][0]), lo(v[0]));
+    s = fma2(hi(T[0][0]), hi(v[0]), s);
+    float2 t01 = mul2(lo(T[1][0]), lo(v[0])), t23 = mul2(hi(T[1][0]), hi(v[0]));
+    float2 sz = mul2(splat(z), add2(t01, t23));
+#pragma unroll
+    for (int k = 1; k < kRun; k++) {
+      s = fma2(lo(T[0][k]), lo(v[k]), s);
+      s = fma2(hi(T[0][k]), hi(v[k]), s);
+      const float2 a = mul2(lo(T[1][k]), lo(v[k])), b = mul2(hi(T[1][k]), hi(v[k]));
+      sz = fma2(splat(fmaf(p.hzf, float(k), z)), add2(a, b), sz);
+      t01 = add2(t01, a);
+      t23 = add2(t23, b);
+    }
+    const float2 x01 = make_float2(x, x + p.hxf);
+    const float2 x23 = make_float2(fmaf(p.hxf, 2.f, x), fmaf(p.hxf, 3.f, x));
+    const float2 sx = fma2(x01, t01, mul2(x23, t23)), t = add2(t01, t23);
+    c[0] = s.x + s.y;
+    c[1] = y * (t.x + t.y);
+    c[2] = sz.x + sz.y;
+    c[3] = sx.x + sx.y;
+  }
+  static __device__ __forceinline__ void scatter(const LanczosParams &p, const float4 (&T)[nch][kRun],
+                                                 float4 (&u)[kRun], float x, float y, float z,
+                                                 const float (&q)[nlm]) {
+    const float2 q0 = splat(q[0]), qx = splat(q[3]), yz = splat(fmaf(q[1], y, q[2] * z));
+    const float2 x01 = make_float2(x, x + p.hxf);
+    const float2 x23 = make_float2(fmaf(p.hxf, 2.f, x), fmaf(p.hxf, 3.f, x));
+    const float2 g01 = fma2(qx, x01, yz), g23 = fma2(qx, x23, yz);
+    const float qzh = q[2] * p.hzf;
+#pragma unroll
+    for (int k = 0; k < kRun; k++) {
+      const float2 dz = splat(qzh * float(k));
+      const float2 a = k ? add2(g01, dz) : g01, b = k ? add2(g23, dz) : g23;
+      const float2 u01 = fma2(lo(T[1][k]), a, fma2(lo(T[0][k]), q0, lo(u[k])));
+      const float2 u23 = fma2(hi(T[1][k]), b, fma2(hi(T[0][k]), q0, hi(u[k])));
+      u[k] = make_float4(u01.x, u01.y, u23.x, u23.y);
+    }
+  }
+};
+
+// Planes [a, b) of an item's column that an image's support meets.
+struct ListRun {
+  int a, b;
+  __device__ __forceinline__ int units() const { return (max(b - a, 0) + kRun - 1) / kRun; }
+};
+// Item t of the list: chunk t / columns of column t % columns.
+struct ListItem {
+  int column;   // quad index in a plane
+  int zb, ze;   // its planes, from the first owned one
+  int top;      // units end here: ze, or kRun in a cube of fewer planes (that many are allocated)
+  float x, y;   // cube coordinates of the column's first point
+  __device__ __forceinline__ ListItem(int t, int columns, int chunks, int nq, int planes) {
+    const int chunk = t / columns;
+    column = t - chunk * columns;
+    const int row = column / nq;
+    x = float(4 * (column - row * nq));
+    y = float(row);
+    zb = planes * chunk / chunks;
+    ze = planes * (chunk + 1) / chunks;
+    top = max(ze, zb + kRun);
+  }
+  __device__ __forceinline__ ListRun run(const LanczosParams &p, const ImgRow *row, int nx, float ih) const {
+    const ImgRow g = load_row(row);
+    const TypeDesc &td = p.types[g.type];
+    const float fx = x - g.bx, fy = y - g.by;
+    float near = 3e38f;  // smallest dx^2 of the points in the cube and the box
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const float f = fx + float(i), dx = fmaf(p.hxf, f, g.ox);
+      if (f >= 0.f && f < float(td.fx) && x + float(i) < float(nx)) near = fminf(near, dx * dx);
+    }
+    const float dy = fmaf(p.hyf, fy, g.oy), rest = td.support_r2_f32 - near - dy * dy;
+    if (!(rest >= 0.f) || fy < 0.f || fy >= float(td.fy)) return ListRun{0, 0};
+    // |oz + hz (z - bz)| <= sqrt(rest), a touch wider: T is masked point by point
+    const float half = sqrtf(rest);
+    const float low = fmaf(-half - g.oz, ih, -1e-3f), high = fmaf(half - g.oz, ih, 1e-3f);
+    const int bz = (int)g.bz;
+    ListRun r;
+    r.a = max(zb, bz + max(0, (int)ceilf(low)));
+    r.b = min(ze, bz + min(td.fz, (int)floorf(high) + 1));
+    return r.b > r.a ? r : ListRun{0, 0};
+  }
+};
+// Exclusive scan of n integers in place by one warp; returns their sum.
+__device__ __forceinline__ int warp_exclusive_scan(int *v, int n) {
+  const int lane = threadIdx.x & 31;
+  const int per = (n + 31) / 32, b = min(n, lane * per), e = min(n, b + per);
+  int sum = 0;
+  for (int i = b; i < e; i++) sum += v[i];
+  int incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  int at = incl - sum;
+  for (int i = b; i < e; i++) {
+    const int t = v[i];
+    v[i] = at;
+    at += t;
+  }
+  __syncwarp();
+  return __shfl_sync(0xffffffffu, incl, 31);
 }
-template <int N>
-__device__ __forceinline__ void rec_load_keep(const float4 *rec, int e, float *c,
-                                              unsigned long long pol) {
-  constexpr int nv = (N + 3) / 4;
+
+// Sum of N values over the warp; the total of value i goes to fn(i, total) in one lane.  N = 4 halves
+// the values with the lanes first (6 shuffles instead of 20).
+template <int N, typename FN> __device__ __forceinline__ void warp_totals(const float (&v)[N], FN &&fn) {
+  const int lane = threadIdx.x & 31;
+  if constexpr (N == 4) {
+    const bool h16 = lane & 16, h8 = lane & 8;
+    float a = h16 ? v[2] : v[0], b = h16 ? v[3] : v[1];
+    a += __shfl_xor_sync(0xffffffffu, h16 ? v[0] : v[2], 16);
+    b += __shfl_xor_sync(0xffffffffu, h16 ? v[1] : v[3], 16);
+    float c = h8 ? b : a;
+    c += __shfl_xor_sync(0xffffffffu, h8 ? a : b, 8);
 #pragma unroll
-  for (int j = 0; j < nv; j++) {
-    const float4 x = ld_keep(rec + (size_t)e * nv + j, pol);
-    const float t[4] = {x.x, x.y, x.z, x.w};
+    for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    if ((lane & 7) == 0) fn(lane >> 3, c);
+  } else {
 #pragma unroll
-    for (int q = 0; q < 4; q++)
-      if (4 * j + q < N) c[4 * j + q] = t[q];
+    for (int s = 0; s < N; s++) {
+      const float r = lk::warp_sum(v[s]);
+      if (lane == 0) fn(s, r);
+    }
   }
 }
 
@@ -293,12 +522,10 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
                                           unsigned char *proj_scratch, double *__restrict__ ab_out,
                                           int *__restrict__ status) {
   constexpr int NLM = lk::Lm<MASK>::nlm;
-  using Rec = lk::ProjRec<float, NLM>;
-  // points per lane per batch of the gather and of the scatter (all loads of a batch are in
-  // flight together; larger batches waste more lanes at the end of each image's range)
-  constexpr int kRecBytes = Rec::nvec * (int)sizeof(typename Rec::vec_t);
-  constexpr int kStreamG = kRecBytes <= 16 ? 6 : lk::stream_batch<kRecBytes>();
-  constexpr int kStreamS = kRecBytes <= 16 ? 8 : lk::stream_batch<kRecBytes>();
+  using Chi = UnitChi<MASK>;
+  constexpr int NCH = Chi::nch;
+  constexpr int kTCols = 4 * kRun * NCH;  // tensor-memory columns of a unit's T
+  constexpr int kPart = (NLM + 3) / 4;    // float4 of a unit's partial sums
   const int nw = blockDim.x >> 5;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nx = p.nx, ny = p.ny, nz = p.nz, pitch = p.pitch;
@@ -312,10 +539,9 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
   if constexpr (PAIR) cr = (int)cooperative_groups::this_cluster().block_rank();
   const PairPlanes pp = PAIR ? pair_planes(nz, p.zsplit, cr) : PairPlanes{0, nz, 0, nz};
   const int zo0 = pp.zo0, zo1 = pp.zo1, pz0 = pp.pz0, pz1 = pp.pz1, nzo = zo1 - zo0;
-  const int ncp = (PAIR ? pair_p_planes(nz, p.zsplit) : nz) * PS;  // floats of P
-  const int ncu = (PAIR ? pair_u_planes(nz, p.zsplit) : nz) * PS;  // floats of U
+  const int ncp = (PAIR ? pair_p_planes(nz, p.zsplit) : list_planes(nz)) * PS;  // floats of P
+  const int ncu = (PAIR ? pair_u_planes(nz, p.zsplit) : list_planes(nz)) * PS;  // floats of U
   const int pofs4 = -pz0 * PS4, uofs4 = -zo0 * PS4;  // quad index shifts of planes
-  const int udelta = (zo0 - pz0) * PS;  // U index of a list point = its P index - udelta
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float *P = reinterpret_cast<float *>(smem_raw);
@@ -326,10 +552,6 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
   float2 *red_a = sum_b + 64;  // per-warp double-float partials
   float2 *red_b = red_a + kMaxWarps;
   cur += sizeof(float2) * (2 * kMaxWarps + 128);
-  // gathered c per (warp, image): warp w's range covers images k_first(w).. so k + w is
-  // unique for every pair it visits; plain stores, summed per slot in a fixed order
-  float *part = reinterpret_cast<float *>(cur);
-  cur += sizeof(float) * (maxi + kMaxWarps) * NLM;
   float *alpha = reinterpret_cast<float *>(cur);
   cur += sizeof(float) * maxi * NLM;
   // PAIR: the two CTAs' gathered c per (slot, lm), [rank][slot * NLM + lm] (each CTA writes
@@ -347,33 +569,40 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
     cur += sizeof(int) * 4;
   }
   int *img = reinterpret_cast<int *>(cur);
-  int *slot = img + maxi;
-  int *slot_type = slot + maxi;
-  int *blo = slot_type + maxi;
-  int *bext = blo + maxi;
-  int *pref = bext + maxi;      // maxi + 1
-  int *kept = pref + maxi + 1;
-  int *koff = kept + maxi;      // maxi + 1
-  int *slot_first = koff + maxi + 1;  // first image of every slot (images sorted by atom)
-  int *cnt = slot_first + maxi;  // [0] images, [1] slots, [2] overflow, [3] next node
+  int *slot_type = img + maxi;
+  int *slot_first = slot_type + maxi;    // first image of every slot (images sorted by atom), n_img
+  int *slot_base = slot_first + maxi + 1;  // first partial sums of every slot, their number
+  int *cnt = slot_base + maxi + 1;  // [0] images, [1] slots, [2] overflow, [3] next node, [4] TMEM, [5] most units
+  int *wunits = cnt + 6;            // units of every warp's longest lane
+  ImgRow *rows = reinterpret_cast<ImgRow *>(
+      (reinterpret_cast<uintptr_t>(wunits + kMaxWarps) + 15) & ~static_cast<uintptr_t>(15));
+  float4 *zq = reinterpret_cast<float4 *>(rows + maxi);  // a quad of zeros
+  float4 *part_s = zq + 1;                               // [p.part_cap] partial sums
+  // scratch of the list build: U, which is cleared after it, if it is large enough
+  int *scratch = list_scratch_bytes(maxi, nw) <= 4 * ncu ? reinterpret_cast<int *>(U)
+                                                         : reinterpret_cast<int *>(part_s + p.part_cap);
 
-  typename Rec::vec_t *rec = reinterpret_cast<typename Rec::vec_t *>(
-      proj_scratch + (size_t)blockIdx.x * p.proj_bytes_per_cta);
-  unsigned *ridx = reinterpret_cast<unsigned *>(
-      reinterpret_cast<unsigned char *>(rec) + (size_t)p.proj_cap * sizeof(typename Rec::vec_t) * Rec::nvec);
+  // this CTA's slice of global scratch: T of the units beyond the tensor memory and all unit words
+  // (both [batch][lane]), partial sums
+  float4 *gT = reinterpret_cast<float4 *>(proj_scratch + (size_t)blockIdx.x * p.proj_bytes_per_cta);
+  unsigned *gword = reinterpret_cast<unsigned *>(gT + (size_t)p.list_batches * 32 * kRun * NCH);
+  float4 *part_g = reinterpret_cast<float4 *>(gword + (size_t)p.list_batches * 32);
 
   float4 *P4 = reinterpret_cast<float4 *>(P);
   float4 *U4 = reinterpret_cast<float4 *>(U);
+  float4 *P4o = P4 + (zo0 - pz0) * PS4;  // the owned planes of P, indexed as U
   const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
   // byte addresses: P, U, a quad of zeros that stands for every plane and row outside the cube
   const unsigned sP = smem_addr(P), sU = smem_addr(U);
-  float4 *zq = reinterpret_cast<float4 *>(
-      (reinterpret_cast<uintptr_t>(cnt + 4) + 15) & ~static_cast<uintptr_t>(15));
   const unsigned sZ = smem_addr(zq);
   if (threadIdx.x == 0) *zq = zero4;  // the node loop's first barrier comes before its first use
   const int PB = 16 * PS4, RB = 16 * nq;  // bytes of a plane and of a row
-  const unsigned long long kpol = l2_keep_policy();
-  static_assert(std::is_same<typename Rec::vec_t, float4>::value, "FP32 records of float4");
+  // list items: column (quad xq of row y) and plane range [nzo c / nlc, nzo (c+1) / nlc) of the owned
+  const int ncol = nq * ny, nlc = list_chunks(ncol, nzo, blockDim.x), n_item = ncol * nlc;
+  if (warp == 0) tc5::tmem_alloc(reinterpret_cast<uint32_t *>(cnt + 4), kListColumns);
+  __syncthreads();
+  const float ihz = 1.f / p.hzf;
+  const unsigned tquarter = (unsigned)cnt[4] + ((unsigned)(warp & 3) << 21);  // the warp's lanes
 
   // thread -> quad of a row (pass A) / of a plane (pass B): nq consecutive threads own the
   // quads of one row or plane, so consecutive threads touch consecutive 16-byte quads
@@ -407,7 +636,7 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
     const int K = (int)(node / ((long long)p.Nx * p.Ny));
     const int Xs = I - p.nhx, Ys = J - p.nhy, Zs = K - p.nhz;
 
-    // ---- per-node image list, slots and point offsets (warp 0); others clear ----
+    // ---- per-node image list and slots (warp 0); others clear P ----
     if (warp == 0) {
       int count = 0;
       for (int base = 0; base < p.n_images; base += 32) {
@@ -426,59 +655,102 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
       }
       __syncwarp();
       const int n = min(count, maxi);
-      int slots = 0, offset = 0;
+      int slots = 0;
       for (int base = 0; base < n; base += 32) {
         const int k = base + lane;
         bool start = false;
-        int npts = 0, lo = 0, ext = 0, atom = -1, type = 0;
+        ImageMeta m{};
         if (k < n) {
-          const ImageMeta m = images[img[k]];
-          atom = m.atom;
-          type = m.type;
-          start = (k == 0) || images[img[k - 1]].atom != atom;
-          const TypeDesc &td = p.types[m.type];
-          const int xa = max(m.bx, Xs), ya = max(m.by, Ys), za = max(m.bz, Zs + zo0);
-          const int ex = min(m.bx + td.fx, Xs + nx) - xa;
-          const int ey = min(m.by + td.fy, Ys + ny) - ya;
-          const int ez = max(0, min(m.bz + td.fz, Zs + zo1) - za);  // owned planes only
-          npts = ex * ey * ez;
-          lo = (xa - Xs) | ((ya - Ys) << 10) | ((za - Zs) << 20);
-          ext = ex | (ey << 10) | (ez << 20);
+          m = images[img[k]];
+          start = (k == 0) || images[img[k - 1]].atom != m.atom;
         }
-        const unsigned m = __ballot_sync(0xffffffffu, start);
-        const int g = slots + __popc(m & ((1u << lane) - 1u)) + (start ? 0 : -1);
-        int incl = npts;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int t = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= o) incl += t;
-        }
+        const unsigned starts = __ballot_sync(0xffffffffu, start);
+        const int g = slots + __popc(starts & ((1u << lane) - 1u)) + (start ? 0 : -1);
         if (k < n) {
-          slot[k] = g;
+          rows[k] = ImgRow{(float)(m.bx - Xs), (float)(m.by - Ys), (float)(m.bz - Zs - zo0), (float)m.ox,
+                           (float)m.oy,        (float)m.oz,        m.type,                   g};
           if (start) {
-            slot_type[g] = type;
+            slot_type[g] = m.type;
             slot_first[g] = k;
           }
-          blo[k] = lo;
-          bext[k] = ext;
-          pref[k] = offset + incl - npts;
         }
-        slots += __popc(m);
-        offset += __shfl_sync(0xffffffffu, incl, 31);
+        slots += __popc(starts);
       }
       if (lane == 0) {
-        pref[n] = offset;
+        slot_first[slots] = n;
         cnt[0] = n;
         cnt[1] = slots;
         cnt[2] = count > maxi;
+        cnt[5] = 0;
       }
     } else {
       for (int e = threadIdx.x - 32; e < (ncp >> 2); e += blockDim.x - 32) P4[e] = zero4;
-      for (int e = threadIdx.x - 32; e < (ncu >> 2); e += blockDim.x - 32) U4[e] = zero4;
     }
     __syncthreads();
     const int n_img = cnt[0], n_slot = cnt[1];
-    bool overflow = cnt[2] || pref[n_img] > p.proj_cap;
+
+    // ---- items dealt to the threads by their number of units, the most first ----
+    int *hist = scratch, *order = scratch + kSortKeys * nw, *kw = order + 32 * nw;
+    int units = 0;
+    if (threadIdx.x < n_item) {
+      const ListItem it(threadIdx.x, ncol, nlc, nq, nzo);
+      for (int k = 0; k < n_img; k++) units += it.run(p, rows + k, nx, ihz).units();
+    }
+    const int most = __reduce_max_sync(0xffffffffu, units);
+    if (lane == 0) atomicMax(cnt + 5, most);
+    __syncthreads();
+    {
+      int shift = 0;
+      while ((cnt[5] >> shift) >= kSortKeys) shift++;
+      // key kSortKeys - 1 - units (threads without an item last); every warp's count per key
+      const int key = threadIdx.x < n_item ? kSortKeys - 1 - (units >> shift) : kSortKeys - 1;
+      unsigned mine = 0;
+      for (int q = 0; q < kSortKeys; q += 32) {
+        int c = 0;
+        for (int v = 0; v < 32; v++) {
+          const unsigned m = __ballot_sync(0xffffffffu, key == q + v);
+          if (key == q + v) mine = m;
+          if (lane == v) c = __popc(m);
+        }
+        hist[(q + lane) * nw + warp] = c;
+      }
+      __syncthreads();
+      if (warp == 0) warp_exclusive_scan(hist, kSortKeys * nw);
+      __syncthreads();
+      order[hist[key * nw + warp] + __popc(mine & ((1u << lane) - 1u))] = threadIdx.x;
+    }
+    __syncthreads();
+    const int my = order[threadIdx.x];
+    const bool has_item = my < n_item;
+    const ListItem item(has_item ? my : 0, ncol, nlc, nq, nzo);
+    units = 0;
+    for (int k = 0; k < n_img; k++) {  // units per image of every warp
+      const int u = has_item ? item.run(p, rows + k, nx, ihz).units() : 0;
+      units += u;
+      const int t = __reduce_add_sync(0xffffffffu, u);
+      if (lane == 0) kw[k * nw + warp] = t;
+    }
+    const int w_units = __reduce_max_sync(0xffffffffu, units);
+    if (lane == 0) wunits[warp] = w_units;
+    __syncthreads();
+    if (warp == 0) {
+      const int total = warp_exclusive_scan(kw, n_img * nw);
+      for (int g = lane; g < n_slot; g += 32) slot_base[g] = kw[slot_first[g] * nw];
+      if (lane == 0) slot_base[n_slot] = total;
+    }
+    // batches (units of a warp's 32 lanes) before this warp's, and units before it in its quarter
+    int batch0 = 0, batches = 0, quarter0 = 0;
+    for (int w = 0; w < nw; w++) {
+      const int u = wunits[w];
+      if (w < warp) {
+        batch0 += u;
+        if ((w & 3) == (warp & 3)) quarter0 += u;
+      }
+      batches += u;
+    }
+    __syncthreads();
+    const int n_part = slot_base[n_slot];
+    bool overflow = cnt[2] || batches > p.list_batches || n_part > p.part_total;
     if constexpr (PAIR) {  // both CTAs take the capacity branch together
       if (threadIdx.x == 0) {
         xflag[cr] = overflow;
@@ -500,86 +772,116 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
       else __syncthreads();
       continue;
     }
-    {  // v_0: the unit vector at the cube centre, in every CTA that holds that plane of P
-      const int zc = (nz - 1) / 2;
-      if (threadIdx.x == 0 && zc >= pz0 && zc < pz1)
-        P[(zc - pz0) * PS + (ny - 1) / 2 * pitch + (nx - 1) / 2] = 1.f;
-    }
+    float4 *part = n_part * kPart <= p.part_cap ? part_s : part_g;
+    const int tm_units = max(0, min(w_units, list_units_per_quarter(NCH) - quarter0));
+    const unsigned tmT = tquarter + (unsigned)(quarter0 * kTCols);
+    const unsigned tmW = tquarter + (unsigned)(kListColumns - kListHeads + quarter0);
+    float4 *wT = gT + (size_t)batch0 * 32 * kRun * NCH + lane;  // of unit u: + ((u * NCH + c) * kRun + k) * 32
+    unsigned *wword = gword + (size_t)batch0 * 32 + lane;       // of unit u: + u * 32
 
-    // ---- this node's projector list: one warp per image, support points only ----
-    for (int kk = warp; kk < n_img; kk += nw) {
-      const lk::ImgView<float> v =
-          lk::load_view<float>(p, images, tables, img[kk], blo[kk], bext[kk], Xs, Ys, Zs, pofs4 * 4, PS);
-      const int npts = pref[kk + 1] - pref[kk];
-      int kept_n = 0;
-      for (int q0 = 0; q0 < npts; q0 += 32) {
-        const int q = q0 + lane;
-        int lx, ly, lz;
-        lk::decode(v, min(q, npts - 1), lx, ly, lz);
-        const float dx = v.ox + p.hxf * float(lx), dy = v.oy + p.hyf * float(ly),
-                    dz = v.oz + p.hzf * float(lz);
-        const bool ok = q < npts && dx * dx + dy * dy + dz * dz <= v.r2max;
-        const unsigned m = __ballot_sync(0xffffffffu, ok);
-        if (ok) {
-          const float *tb = v.tab + lz * v.fxy + ly * v.fx + lx;
-          float out[Rec::n];
-#pragma unroll
-          for (int s = 0; s < Rec::n; s++) out[s] = 0.f;
-          int chan = 0;
-          auto channel = [&](auto Lc) {
-            constexpr int L = decltype(Lc)::value;
-            if constexpr (MASK & (1 << L)) {
-              if (v.chan_mask & (1 << L)) {
-                const float t = tb[(chan++) * v.fvol];
-                lk::solid_harmonics<L, float>(dx, dy, dz, [&](int s, float ylm) {
-                  out[lk::Lm<MASK>::rank(s)] = ylm * t;
-                });
-              }
-            }
-          };
-          channel(std::integral_constant<int, 0>{});
-          channel(std::integral_constant<int, 1>{});
-          channel(std::integral_constant<int, 2>{});
-          channel(std::integral_constant<int, 3>{});
-          const int e = pref[kk] + kept_n + __popc(m & ((1u << lane) - 1u));
-          rec_store_keep<NLM>(rec, e, out, kpol);
-          st_keep(ridx + e, (unsigned)(v.pbase + lz * PS + ly * pitch + lx), kpol);
-        }
-        kept_n += __popc(m);
-      }
-      if (lane == 0) kept[kk] = kept_n;
-    }
-    __syncthreads();
-    if (warp == 0) {  // exclusive scan of kept -> koff
-      int offset = 0;
-      for (int base = 0; base < n_img; base += 32) {
-        const int kk = base + lane;
-        const int c = kk < n_img ? kept[kk] : 0;
-        int incl = c;
+    // ---- the units' words, then their T ----
+    {
+      int u = 0;
+      for (int k = 0; k < n_img; k++) {
+        const ListRun r = has_item ? item.run(p, rows + k, nx, ihz) : ListRun{0, 0};
+        const int n = r.units();
+        int incl = n;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
           const int t = __shfl_up_sync(0xffffffffu, incl, o);
           if (lane >= o) incl += t;
         }
-        if (kk < n_img) koff[kk] = offset + incl - c;
-        offset += __shfl_sync(0xffffffffu, incl, 31);
+        const int place = kw[k * nw + warp] + incl - n;
+        for (int j = 0; j < n; j++)
+          wword[32 * u++] = unit_word(k, min(r.a + kRun * j, item.top - kRun), place + j);
       }
-      if (lane == 0) koff[n_img] = offset;
+      for (; u < w_units; u++) wword[32 * u] = unit_word(0, item.zb, 0);
+    }
+    __syncwarp();
+    {
+      int prev = -1, covered = 0;  // planes of the image's run that the units before this one cover
+      for (int u = 0; u < w_units; u++) {
+        const unsigned w = wword[32 * u];
+        const int k = (int)(w & 1023), z0 = (int)((w >> 10) & 63);
+        float4 T[NCH][kRun];
+#pragma unroll
+        for (int c = 0; c < NCH; c++)
+#pragma unroll
+          for (int i = 0; i < kRun; i++) T[c][i] = zero4;
+        if (u < units) {
+          const ListRun r = item.run(p, rows + k, nx, ihz);
+          if (k != prev) covered = r.a;
+          prev = k;
+          const ImgRow g = load_row(rows + k);
+          const TypeDesc &td = p.types[g.type];
+          const int fx = td.fx, lx = (int)(item.x - g.bx), ly = (int)(item.y - g.by);
+          const float *tab = tables + images[img[k]].tab_base + (ly * fx + lx);
+          const int fxy = fx * td.fy, fvol = fxy * td.fz;
+          const float dx = fmaf(p.hxf, item.x - g.bx, g.ox), dy = fmaf(p.hyf, item.y - g.by, g.oy);
+#pragma unroll
+          for (int i = 0; i < kRun; i++) {
+            const int z = z0 + i, lz = z - (int)g.bz;
+            const float dz = fmaf(p.hzf, float(z) - g.bz, g.oz), r2yz = fmaf(dy, dy, dz * dz);
+            const bool inz = z >= covered && z < r.b;
+            float v[NCH][4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+              const float x = fmaf(p.hxf, float(q), dx);
+              const bool in = inz && lx + q >= 0 && lx + q < fx && (int)item.x + q < nx &&
+                              fmaf(x, x, r2yz) <= td.support_r2_f32;
+              int c = 0, ch = 0;
+#pragma unroll
+              for (int l = 0; l < 4; l++) {
+                if (!(MASK & (1 << l))) continue;
+                const bool have = td.chan_mask & (1 << l);
+                v[c][q] = in && have ? tab[lz * fxy + ch * fvol + q] : 0.f;
+                ch += have ? 1 : 0;
+                c++;
+              }
+            }
+#pragma unroll
+            for (int c = 0; c < NCH; c++) T[c][i] = make_float4(v[c][0], v[c][1], v[c][2], v[c][3]);
+          }
+          covered = z0 + kRun;
+        }
+        __syncwarp();
+        if (u < tm_units) {
+#pragma unroll
+          for (int c = 0; c < NCH; c++) tmem_st16(tmT + (unsigned)(u * kTCols + 16 * c), T[c]);
+          tmem_st1(tmW + (unsigned)u, w);
+        } else {
+#pragma unroll
+          for (int c = 0; c < NCH; c++)
+#pragma unroll
+            for (int i = 0; i < kRun; i++) wT[((u * NCH + c) * kRun + i) * 32] = T[c][i];
+        }
+      }
+      tmem_wait_st();
+    }
+    auto load_unit = [&](int u, float4 (&T)[NCH][kRun], unsigned &w) {
+      if (u < tm_units) {
+#pragma unroll
+        for (int c = 0; c < NCH; c++) tmem_ld16(tmT + (unsigned)(u * kTCols + 16 * c), T[c]);
+        tmem_ld1(tmW + (unsigned)u, w);
+        tmem_wait_ld(T, w);
+      } else {
+        w = wword[32 * u];
+#pragma unroll
+        for (int c = 0; c < NCH; c++)
+#pragma unroll
+          for (int i = 0; i < kRun; i++) T[c][i] = wT[((u * NCH + c) * kRun + i) * 32];
+      }
+    };
+    // the item's column in P (owned planes) and U
+    const unsigned itemP = smem_addr(P4o) + 16u * (unsigned)item.column, itemU = sU + 16u * (unsigned)item.column;
+    __syncthreads();  // the scratch in U is read
+    for (int e = threadIdx.x; e < (ncu >> 2); e += blockDim.x) U4[e] = zero4;
+    {  // v_0: the unit vector at the cube centre, in every CTA that holds that plane of P
+      const int zc = (nz - 1) / 2;
+      if (threadIdx.x == 0 && zc >= pz0 && zc < pz1)
+        P[(zc - pz0) * PS + (ny - 1) / 2 * pitch + (nx - 1) / 2] = 1.f;
     }
     __syncthreads();
-    const int total = koff[n_img];
-    const int per = (total + nw - 1) / nw;
-    const int r_begin = min(total, warp * per), r_end = min(total, r_begin + per);
-    int k_first = 0;  // image holding kept point r_begin: largest k with koff[k] <= r_begin
-    {
-      int lo = 0, hi = n_img;
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (koff[mid] <= r_begin) lo = mid;
-        else hi = mid - 1;
-      }
-      k_first = min(lo, max(n_img - 1, 0));
-    }
 
     // quad-aligned copy of the padded Veff + cdiag for this node (copy s: I + s = 0 mod 4)
     const int sh = (4 - (I & 3)) & 3;
@@ -596,38 +898,27 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
       const float2 sc2 = splat(sc), ngh2 = splat(-gam.hi), ngl2 = splat(-gam.lo);
 
       // ---- phase 1: projector gather  ||  pass A ----
-      {
-        int pos = r_begin, k = k_first;
-        while (pos < r_end) {
-          const int kend = min(r_end, koff[k + 1]);
-          const int shift = pref[k] - koff[k];
-          float acc[NLM];
+      for (int u = 0; u < w_units; u++) {
+        float4 T[NCH][kRun];
+        unsigned w;
+        load_unit(u, T, w);
+        const ImgRow g = load_row(rows + (w & 1023u));
+        const int z0 = (int)((w >> 10) & 63u);
+        unsigned a = itemP + (unsigned)(z0 * PB);
+        float4 v[kRun];
 #pragma unroll
-          for (int s = 0; s < NLM; s++) acc[s] = 0.f;
-          for (int i0 = pos + lane; i0 < kend; i0 += 32 * kStreamG) {
-            float c[kStreamG][NLM];
-            unsigned ix[kStreamG];
+        for (int i = 0; i < kRun; i++, a += (unsigned)PB) v[i] = lds_quad(a);
+        float c[NLM];
+        Chi::gather(p, T, v, fmaf(p.hxf, item.x - g.bx, g.ox), fmaf(p.hyf, item.y - g.by, g.oy),
+                    fmaf(p.hzf, float(z0) - g.bz, g.oz), c);
+        if (u < units) {
+          float4 *dst = part + (size_t)(w >> 16) * kPart;
 #pragma unroll
-            for (int u = 0; u < kStreamG; u++) {
-              const int e = min(i0 + 32 * u, kend - 1) + shift;
-              ix[u] = ld_keep(ridx + e, kpol);
-              rec_load_keep<NLM>(rec, e, c[u], kpol);
-            }
-#pragma unroll
-            for (int u = 0; u < kStreamG; u++) {
-              const float val = (i0 + 32 * u < kend) ? P[ix[u]] : 0.f;
-#pragma unroll
-              for (int s = 0; s < NLM; s++) acc[s] = fmaf(c[u][s], val, acc[s]);
-            }
-          }
-#pragma unroll
-          for (int s = 0; s < NLM; s++) {
-            const float r = lk::warp_sum(acc[s]);
-            if (lane == 0) part[(k + warp) * NLM + s] = r;
-          }
-          pos = kend;
-          k++;
+          for (int i = 0; i < kPart; i++)
+            dst[i] = make_float4(c[4 * i], 4 * i + 1 < NLM ? c[4 * i + 1] : 0.f,
+                                 4 * i + 2 < NLM ? c[4 * i + 2] : 0.f, 4 * i + 3 < NLM ? c[4 * i + 3] : 0.f);
         }
+        __syncwarp();
       }
       Kahan ka;
       if (actA) {
@@ -769,28 +1060,38 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
           }
         }
       }
-      // alpha = Gamma_l s c, with c = <chi, P>; <P, V_nl P> = sum Gamma_l c^2 joins the a_k sum
-      for (int e = threadIdx.x; e < n_slot * NLM; e += blockDim.x) {
-        const int sl = e / NLM, r = e - sl * NLM;
-        const TypeDesc &td = p.types[slot_type[sl]];
-        const int l = p.rank_l[r];
-        // c of the slot: its images' partials from every warp whose range meets them, in a
-        // fixed order (no atomics: shared-memory float atomics on a few hot addresses stall)
-        float csum = 0.f;
-        for (int k = slot_first[sl]; k < n_img && slot[k] == sl; k++) {
-          if (koff[k + 1] == koff[k]) continue;
-          const int w1 = (koff[k + 1] - 1) / per;
-          for (int w = koff[k] / per; w <= w1; w++) csum += part[(k + w) * NLM + r];
+      // c of every slot, its units' partial sums in a fixed order, one warp per slot; alpha =
+      // Gamma_l s c (the harmonics' constants on both sides), <P, V_nl P> = sum Gamma_l c^2
+      for (int sl = warp; sl < n_slot; sl += nw) {
+        float c[NLM];
+#pragma unroll
+        for (int s = 0; s < NLM; s++) c[s] = 0.f;
+        for (int j = slot_base[sl] + lane; j < slot_base[sl + 1]; j += 32) {
+#pragma unroll
+          for (int i = 0; i < kPart; i++) {
+            const float4 t = part[(size_t)j * kPart + i];
+            c[4 * i] += t.x;
+            if (4 * i + 1 < NLM) c[4 * i + 1] += t.y;
+            if (4 * i + 2 < NLM) c[4 * i + 2] += t.z;
+            if (4 * i + 3 < NLM) c[4 * i + 3] += t.w;
+          }
         }
-        if constexpr (PAIR) {  // this CTA's part of c, into both CTAs' row cr of cx
-          cx[cr * maxi * NLM + e] = csum;
-          *cooperative_groups::this_cluster().map_shared_rank(cx + cr * maxi * NLM + e, cr ^ 1) = csum;
-        } else {
-          const float gl = (td.chan_mask & (1 << l)) ? float(td.gamma[l]) : 0.f;
-          const float al = gl * csum;
-          alpha[e] = al * sc;
-          ka.add(al * csum);
-        }
+        __syncwarp();
+        warp_totals<NLM>(c, [&](int r, float total) {
+          const float cr_sum = total * Chi::norm(r);
+          if constexpr (PAIR) {  // this CTA's part of c, into both CTAs' row cr of cx
+            float *x = cx + cr * maxi * NLM + sl * NLM + r;
+            *x = cr_sum;
+            *cooperative_groups::this_cluster().map_shared_rank(x, cr ^ 1) = cr_sum;
+          } else {
+            const TypeDesc &td = p.types[slot_type[sl]];
+            const int l = p.rank_l[r];
+            const float gl = (td.chan_mask & (1 << l)) ? float(td.gamma[l]) : 0.f;
+            const float al = gl * cr_sum;
+            alpha[sl * NLM + r] = al * sc * Chi::norm(r);
+            ka.add(al * cr_sum);
+          }
+        });
       }
       {
         const DF ap = df_warp_sum(df_of(ka));
@@ -800,51 +1101,9 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
       else __syncthreads();
 
       // ---- phase 3: projector scatter U += chi alpha  ||  a_k ----
-      {
-        int pos = r_begin, k = k_first;
-        while (pos < r_end) {
-          const int kend = min(r_end, koff[k + 1]);
-          const int shift = pref[k] - koff[k];
-          float coef[NLM];
-          if constexpr (PAIR) {  // alpha = Gamma_l s (c_0 + c_1) from the two CTAs' rows
-            const int sl = slot[k];
-            const TypeDesc &td = p.types[slot_type[sl]];
-#pragma unroll
-            for (int s = 0; s < NLM; s++) {
-              const int l = p.rank_l[s];
-              const float gl = (td.chan_mask & (1 << l)) ? float(td.gamma[l]) : 0.f;
-              coef[s] = gl * ((cx[sl * NLM + s] + cx[maxi * NLM + sl * NLM + s]) * sc);
-            }
-          } else {
-            const float *al = alpha + slot[k] * NLM;
-#pragma unroll
-            for (int s = 0; s < NLM; s++) coef[s] = al[s];
-          }
-          for (int i0 = pos + lane; i0 < kend; i0 += 32 * kStreamS) {
-            float c[kStreamS][NLM];
-            unsigned ix[kStreamS];
-#pragma unroll
-            for (int u = 0; u < kStreamS; u++) {
-              const int e = min(i0 + 32 * u, kend - 1) + shift;
-              ix[u] = ld_keep(ridx + e, kpol);
-              rec_load_keep<NLM>(rec, e, c[u], kpol);
-            }
-#pragma unroll
-            for (int u = 0; u < kStreamS; u++) {
-              float val = 0.f;
-#pragma unroll
-              for (int s = 0; s < NLM; s++) val = fmaf(c[u][s], coef[s], val);
-              // fire-and-forget shared atomics: a plain read-add-write waits on the read
-              if (i0 + 32 * u < kend) atomicAdd(&U[ix[u] - udelta], val);
-            }
-          }
-          pos = kend;
-          k++;
-        }
-      }
-      DF adf;
       if constexpr (PAIR) {
-        // <P, V_nl P> = sum Gamma_l c^2 over the slots, the same sum in both CTAs
+        // alpha from the two CTAs' rows, and <P, V_nl P> = sum Gamma_l c^2 over the slots, the same
+        // sum in both CTAs
         Kahan kn;
         for (int e = threadIdx.x; e < n_slot * NLM; e += blockDim.x) {
           const int sl = e / NLM, r = e - sl * NLM;
@@ -852,11 +1111,33 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
           const int l = p.rank_l[r];
           const float gl = (td.chan_mask & (1 << l)) ? float(td.gamma[l]) : 0.f;
           const float cv = cx[e] + cx[maxi * NLM + e];
+          alpha[e] = gl * cv * sc * Chi::norm(r);
           kn.add(gl * cv * cv);
         }
         const DF np = df_warp_sum(df_of(kn));
         if (lane == 0) red_n[warp] = make_float2(np.hi, np.lo);
         __syncthreads();
+      }
+      for (int u = 0; u < w_units; u++) {
+        float4 T[NCH][kRun];
+        unsigned w;
+        load_unit(u, T, w);
+        const ImgRow g = load_row(rows + (w & 1023u));
+        const int z0 = (int)((w >> 10) & 63u);
+        float q[NLM];
+#pragma unroll
+        for (int s = 0; s < NLM; s++) q[s] = alpha[g.slot * NLM + s];
+        const unsigned a = itemU + (unsigned)(z0 * PB);
+        float4 v[kRun];
+#pragma unroll
+        for (int i = 0; i < kRun; i++) v[i] = lds_quad(a + (unsigned)(i * PB));
+        Chi::scatter(p, T, v, fmaf(p.hxf, item.x - g.bx, g.ox), fmaf(p.hyf, item.y - g.by, g.oy),
+                     fmaf(p.hzf, float(z0) - g.bz, g.oz), q);
+#pragma unroll
+        for (int i = 0; i < kRun; i++) sts_quad_if(u < units, a + (unsigned)(i * PB), v[i]);
+      }
+      DF adf;
+      if constexpr (PAIR) {
         // a_k: CTA 0's stencil partials, CTA 1's, then the projector part (fixed order)
         auto cl = cooperative_groups::this_cluster();
         const float2 *ra0 = cr == 0 ? red_a : cl.map_shared_rank(red_a, 0);
@@ -864,18 +1145,17 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
         adf = df_add(df_add(df_all_reduce(ra0, nw), df_all_reduce(ra1, nw)), df_all_reduce(red_n, nw));
       } else {
         adf = df_all_reduce(red_a, nw);
-        __syncthreads();
       }
+      __syncthreads();
 
       // ---- phase 4: w = U - a_k v, P <- w, U <- v, b_k^2 partial ----
       {
         const DF ak = df_div(adf, n2);
         const float2 nah2 = splat(-ak.hi), nal2 = splat(-ak.lo);
         Kahan kb;
-        // owned planes: P's at quad e + udelta/4, U's at e.  PAIR: quads [h0, h1) are the
+        // owned planes.  PAIR: quads [h0, h1) are the
         // peer's halo planes and also go to its P at e + dpeer.
         const int nown = nzo * PS4;
-        float4 *P4o = P4 + (udelta >> 2);
         int h0 = 0, h1 = 0, dpeer = 0;
         float4 *P4peer = P4;
         if constexpr (PAIR) {
@@ -957,6 +1237,7 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
   }
   // no CTA of a pair leaves while its peer may still read its shared memory
   if constexpr (PAIR) cooperative_groups::this_cluster().sync();
+  if (warp == 0) tc5::tmem_dealloc((unsigned)cnt[4], kListColumns);
 }
 
 template <int MASK, int MAXT, bool ISO>

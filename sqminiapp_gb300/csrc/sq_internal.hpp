@@ -72,6 +72,9 @@ struct LanczosParams {
   int vq_row;              // kLayoutQuad: row length (floats) of the quad-aligned Veff copies
   long long vq_copy_stride;  // kLayoutQuad: floats per quad-aligned Veff copy
   int proj_cap;            // records of one CTA's projector list (max box points of a node)
+  // kLayoutQuad, per node at most: list units, batches of 32 of them; float4 of shared memory for
+  // their partial sums
+  int part_total, list_batches, part_cap;
   long long proj_bytes_per_cta;
   long long node_begin, node_end;
   double hx, hy, hz;

@@ -63,6 +63,13 @@ size_t lanczos_quad_smem_bytes(const LanczosParams &p);
 int lanczos_quad_threads(const LanczosParams &p);
 // threads to launch a single-CTA split-pass kernel with (>= lanczos_quad_threads)
 int lanczos_quad_block(const LanczosParams &p);
+// The kernel's projector list: planes of a unit, plane ranges per column of quads, bytes of a unit and
+// of one CTA's slice of global scratch; and room in shared memory for the units' partial sums (part_cap).
+constexpr int kQuadListRun = 4;
+int lanczos_quad_list_chunks(int columns, int planes, int threads);
+size_t lanczos_quad_unit_bytes(const LanczosParams &p);
+size_t lanczos_quad_list_bytes(const LanczosParams &p);
+void lanczos_quad_place_partials(LanczosParams &p, int smem_optin);
 // kLayoutPair: clusters of two CTAs that fit on the device at once (0 if none)
 int lanczos_quad_pair_clusters(const LanczosParams &p, int block, size_t smem);
 
