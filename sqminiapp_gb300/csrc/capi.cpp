@@ -372,9 +372,9 @@ void plan_engine(sq_handle *h, int smem_optin, int l2_bytes) {
       if (h->opt.tile > 0) break;
     }
     // The lists of all CTAs, were none of them in tensor memory, must stay in L2 (what exceeds it is
-    // streamed from there): units of whole boxes, about half of which the spheres fill.
+    // streamed from there): units of whole boxes, 0.47 of which the spheres fill (27^3 cube).
     auto list_bytes = [&](const sq::LanczosParams &l) {
-      return (double)h->num_sms * 0.6 * l.part_total * (double)sq::lanczos_quad_unit_bytes(l);
+      return (double)h->num_sms * 0.47 * l.part_total * (double)sq::lanczos_quad_unit_bytes(l);
     };
     if (!wide && threads <= sq::kQuadMaxThreads && words &&
         sq::lanczos_quad_smem_bytes(q) <= (size_t)smem_optin &&
@@ -484,6 +484,38 @@ void plan_engine(sq_handle *h, int smem_optin, int l2_bytes) {
   h->info.kernel_smem_bytes = (int)h->smem;
 }
 
+// The split-pass kernel's tables replace the plain ones; its images point into them.
+void use_quad_tables(sq_handle *h) {
+  const sq::Setup &s = h->setup;
+  std::vector<sq::QuadTable> tabs(s.n_tables);
+  std::vector<char> seen(s.n_tables, 0);
+  std::vector<sq::ImageMeta> images(s.images);
+  long long total = 0;
+  for (sq::ImageMeta &im : images) {
+    if (!seen[im.tab]) {
+      seen[im.tab] = 1;
+      tabs[im.tab] = {im.tab_base, total, im.type, (float)im.ox, (float)im.oy, (float)im.oz};
+      total += sq::quad_table_float4(s.types[im.type]);
+    }
+    im.tab_base = tabs[im.tab].dst;
+  }
+  if (total >= 1LL << 31) throw std::invalid_argument("radial tables too large");
+  if (images.empty()) return;
+  sq::DevBuf<sq::QuadTable> d_tabs(sizeof(sq::QuadTable) * tabs.size(), "quad table list");
+  void *quads = nullptr;
+  dev_alloc(&quads, 16 * (size_t)total, "quad tables");
+  void *plain = h->d_tables;
+  h->d_tables = quads;  // owned by the handle from here on
+  sq::DevBuf<void> old(plain);
+  ck(cudaMemcpyAsync(d_tabs.get(), tabs.data(), sizeof(sq::QuadTable) * tabs.size(), cudaMemcpyHostToDevice,
+                     h->own_stream), "quad table list H2D");
+  ck(sq::launch_quad_tables(h->lp, d_tabs.get(), (int)tabs.size(), (const float *)plain, quads, h->own_stream),
+     "quad tables");
+  ck(cudaMemcpyAsync(h->d_images, images.data(), sizeof(sq::ImageMeta) * images.size(), cudaMemcpyHostToDevice,
+                     h->own_stream), "images H2D");
+  ck(cudaStreamSynchronize(h->own_stream), "quad tables");
+}
+
 void build_engine(sq_handle *h) {
   ck(cudaSetDevice(h->opt.device), "cudaSetDevice");
   ck(cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, h->opt.device), "sm count");
@@ -510,6 +542,7 @@ void build_engine(sq_handle *h) {
   if (h->opt.precision == 32) {
     std::vector<float> t32(s.tables.begin(), s.tables.end());
     ck(cudaMemcpy(h->d_tables, t32.data(), 4 * t32.size(), cudaMemcpyHostToDevice), "tables H2D");
+    if (h->quad) use_quad_tables(h);
   } else {
     ck(cudaMemcpy(h->d_tables, s.tables.data(), 8 * s.tables.size(), cudaMemcpyHostToDevice),
        "tables H2D");

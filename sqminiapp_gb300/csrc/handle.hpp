@@ -39,6 +39,7 @@ template <typename P> void dev_free(P *&ptr) {
 template <typename P> struct DevBuf {
   P *p = nullptr;
   DevBuf(size_t bytes, const char *what) { dev_alloc(&p, bytes, what); }
+  explicit DevBuf(P *owned) : p(owned) {}
   ~DevBuf() { dev_free(p); }
   DevBuf(const DevBuf &) = delete;
   DevBuf &operator=(const DevBuf &) = delete;

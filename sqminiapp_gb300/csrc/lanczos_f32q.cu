@@ -33,7 +33,7 @@ size_t lanczos_quad_smem_bytes(const LanczosParams &p) {
       (size_t)(pair ? lq::pair_u_planes(p.nz, p.zsplit) : lq::list_planes(p.nz))};
   size_t b = sizeof(float) * ps * (pu[0] + pu[1]);
   b += sizeof(float2) * (2 * lk::kMaxWarps + 128);           // partials and step sums
-  b += sizeof(float) * (size_t)p.max_img * nlm;              // alpha
+  b += sizeof(float4) * (size_t)p.max_img * ((nlm + 3) / 4);  // alpha
   if (pair)  // both CTAs' c, an 8-byte alignment, projector a_k partials, capacity flags
     b += sizeof(float) * 2 * (size_t)p.max_img * nlm + 8 + sizeof(float) * 2 * lk::kMaxWarps +
          sizeof(int) * 4;
@@ -60,12 +60,13 @@ size_t partial_float4(const LanczosParams &p) { return (mask_nlm(kernel_mask(p.u
 }  // namespace
 
 size_t lanczos_quad_unit_bytes(const LanczosParams &p) {
-  return sizeof(float4) * lq::kRun * channels(p) + sizeof(unsigned);
+  return sizeof(float4) * (lq::kRun * channels(p) + 1);
 }
 
 size_t lanczos_quad_list_bytes(const LanczosParams &p) {
   return (size_t)p.list_batches * 32 * lanczos_quad_unit_bytes(p) +
-         sizeof(float4) * partial_float4(p) * (size_t)p.part_total;
+         sizeof(float4) * partial_float4(p) * (size_t)p.part_total +
+         sizeof(int2) * (size_t)p.max_img * kQuadMaxThreads;  // runs of every item
 }
 
 void lanczos_quad_place_partials(LanczosParams &p, int smem_optin) {
@@ -75,6 +76,42 @@ void lanczos_quad_place_partials(LanczosParams &p, int smem_optin) {
   const size_t room = ((size_t)smem_optin - lanczos_quad_smem_bytes(p)) / sizeof(float4);
   const size_t want = partial_float4(p) * (size_t)(0.6 * p.part_total + 1);
   p.part_cap = (int)std::min(room, want);
+}
+
+// ---- quad tables ----
+long long quad_table_float4(const TypeDesc &td) {
+  return 4LL * __builtin_popcount(td.chan_mask) * lq::quad_table_channel(td);
+}
+
+namespace {
+// One block row per (table, shift, channel): quads of the table's rows behind `shift` zeros, zeros
+// where the point lies outside the support sphere.
+__global__ void quad_tables_kernel(const __grid_constant__ LanczosParams p, const QuadTable *__restrict__ tabs,
+                                   const float *__restrict__ src, float4 *__restrict__ dst) {
+  const QuadTable t = tabs[blockIdx.x];
+  const TypeDesc &td = p.types[t.type];
+  const int row = lq::quad_table_row(td), chan = lq::quad_table_channel(td);
+  const int nch = __popc(td.chan_mask), fvol = td.fx * td.fy * td.fz;
+  for (int e = threadIdx.x + blockDim.x * blockIdx.y; e < 4 * nch * chan; e += blockDim.x * gridDim.y) {
+    const int shift = e / (nch * chan), r = e - shift * nch * chan, c = r / chan, i = r - c * chan;
+    const int q = i % row, ly = i / row % td.fy, lz = i / (row * td.fy);
+    const float dy = fmaf(p.hyf, float(ly), t.oy), dz = fmaf(p.hzf, float(lz), t.oz);
+    float v[4];
+    for (int j = 0; j < 4; j++) {
+      const int lx = 4 * q + j - shift;
+      const float dx = fmaf(p.hxf, float(lx), t.ox);
+      const bool in = lx >= 0 && lx < td.fx && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= td.support_r2_f32;
+      v[j] = in ? src[t.src + (long long)c * fvol + (lz * td.fy + ly) * td.fx + lx] : 0.f;
+    }
+    dst[t.dst + e] = make_float4(v[0], v[1], v[2], v[3]);
+  }
+}
+}  // namespace
+
+cudaError_t launch_quad_tables(const LanczosParams &p, const QuadTable *tabs, int n, const float *src,
+                               void *dst, cudaStream_t s) {
+  quad_tables_kernel<<<dim3(n, 16), 256, 0, s>>>(p, tabs, src, (float4 *)dst);
+  return cudaGetLastError();
 }
 
 size_t veff_quad_floats(const LanczosParams &p) { return 4 * (size_t)p.vq_copy_stride; }

@@ -242,10 +242,10 @@ __host__ __device__ constexpr int pair_u_planes(int nz, int zsplit) {
 // another, zero outside the support and the run.  A thread owns one column of quads over a range of
 // planes ("item") and its units, so no two threads ever meet on a quad.
 constexpr int kRun = 4;
-constexpr int kListColumns = 512;                   // the whole tensor memory of an SM
-constexpr int kListHeads = 32;                      // columns of unit words; the rest holds T_l
-__host__ __device__ constexpr int list_units_per_quarter(int nch) {  // (a quarter: 32 of the 128 lanes)
-  return (kListColumns - kListHeads) / (4 * kRun * nch);
+constexpr int kListColumns = 512;  // the whole tensor memory of an SM
+// Units of a quarter (32 of the 128 lanes): T, the word and (x, y, z) relative to the atom.
+__host__ __device__ constexpr int list_units_per_quarter(int nch) {
+  return kListColumns / (4 * kRun * nch + 4);
 }
 // Plane ranges per column: as many as the threads allow with at least kRun planes each.
 __host__ __device__ constexpr int list_chunks(int columns, int planes, int threads) {
@@ -258,9 +258,16 @@ __host__ __device__ constexpr int list_planes(int planes) {  // planes to alloca
 }
 constexpr int kSortKeys = 64;
 // Bytes of per-node scratch of the list build: a key histogram per warp, the items in order, unit
-// counts per (image, warp).
+// counts per (image, warp), units and runs per item.
 __host__ __device__ constexpr int list_scratch_bytes(int max_img, int nw) {
-  return 4 * (kSortKeys * nw + 32 * nw + max_img * nw);
+  return 4 * (kSortKeys * nw + 32 * nw + max_img * nw + 32 * nw);
+}
+// The radial tables of this kernel hold whole quads: rows of the box's points behind `shift` zeros
+// (four copies, shift 0..3: the image's box start modulo 4 picks the one whose quads are the cube's),
+// zeros outside the support.  Quads of a row, and of a channel.
+__host__ __device__ inline int quad_table_row(const TypeDesc &td) { return (td.fx + 6) / 4; }
+__host__ __device__ inline int quad_table_channel(const TypeDesc &td) {
+  return quad_table_row(td) * td.fy * td.fz;
 }
 
 // Tensor memory: a warp reads and writes its own quarter of the lanes.
@@ -281,18 +288,22 @@ __device__ __forceinline__ void tmem_st16(unsigned taddr, const float4 (&t)[4]) 
       "f"(t[3].w), "r"(taddr)
       : "memory");
 }
-__device__ __forceinline__ void tmem_ld1(unsigned taddr, unsigned &a) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(a) : "r"(taddr));
+__device__ __forceinline__ void tmem_ld4(unsigned taddr, float4 &a) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w)
+               : "r"(taddr));
 }
-__device__ __forceinline__ void tmem_st1(unsigned taddr, unsigned a) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(taddr), "r"(a) : "memory");
+__device__ __forceinline__ void tmem_st4(unsigned taddr, float4 a) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "f"(a.x),
+               "f"(a.y), "f"(a.z), "f"(a.w)
+               : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 // The wait names the registers it guards, so that no use of them moves above it.
-template <int N> __device__ __forceinline__ void tmem_wait_ld(float4 (&t)[N][4], unsigned &w) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(w)::"memory");
+template <int N> __device__ __forceinline__ void tmem_wait_ld(float4 (&t)[N][4], float4 &m) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" : "+f"(m.x), "+f"(m.y), "+f"(m.z), "+f"(m.w)::"memory");
 #pragma unroll
   for (int c = 0; c < N; c++)
 #pragma unroll
@@ -300,18 +311,21 @@ template <int N> __device__ __forceinline__ void tmem_wait_ld(float4 (&t)[N][4],
       asm volatile("" : "+f"(t[c][i].x), "+f"(t[c][i].y), "+f"(t[c][i].z), "+f"(t[c][i].w));
 }
 
-// A unit's word: image (10 bits), first plane from the first owned one (6), place of its partial
+// A unit's word: atom slot (10 bits), first plane from the first owned one (6), place of its partial
 // sums (16).
-__device__ __forceinline__ unsigned unit_word(int image, int z0, int place) {
-  return (unsigned)(image | (z0 << 10)) | ((unsigned)place << 16);
+__device__ __forceinline__ unsigned unit_word(int slot, int z0, int place) {
+  return (unsigned)(slot | (z0 << 10)) | ((unsigned)place << 16);
 }
 // An image of the node: box point 0 in cube coordinates (z from the first owned plane) as floats,
-// its coordinates relative to the atom, type and atom slot.
+// its coordinates relative to the atom, its table (in quads), type and atom slot.
 struct ImgRow {
   float bx, by, bz, ox;
   float oy, oz;
-  int type, slot;
+  int tab, type_slot;
+  __device__ __forceinline__ int type() const { return type_slot & 15; }
+  __device__ __forceinline__ int slot() const { return type_slot >> 4; }
 };
+static_assert(kMaxTypes <= 16, "ImgRow packs the type into 4 bits");
 static_assert(sizeof(ImgRow) == 32, "two 16-byte loads");
 __device__ __forceinline__ ImgRow load_row(const ImgRow *r) {
   const float4 a = reinterpret_cast<const float4 *>(r)[0], b = reinterpret_cast<const float4 *>(r)[1];
@@ -432,12 +446,13 @@ struct ListRun {
 };
 // Item t of the list: chunk t / columns of column t % columns.
 struct ListItem {
-  int column;   // quad index in a plane
+  int index, column;  // t, and the quad index in a plane
   int zb, ze;   // its planes, from the first owned one
   int top;      // units end here: ze, or kRun in a cube of fewer planes (that many are allocated)
   float x, y;   // cube coordinates of the column's first point
   __device__ __forceinline__ ListItem(int t, int columns, int chunks, int nq, int planes) {
     const int chunk = t / columns;
+    index = t;
     column = t - chunk * columns;
     const int row = column / nq;
     x = float(4 * (column - row * nq));
@@ -448,7 +463,7 @@ struct ListItem {
   }
   __device__ __forceinline__ ListRun run(const LanczosParams &p, const ImgRow *row, int nx, float ih) const {
     const ImgRow g = load_row(row);
-    const TypeDesc &td = p.types[g.type];
+    const TypeDesc &td = p.types[g.type()];
     const float fx = x - g.bx, fy = y - g.by;
     float near = 3e38f;  // smallest dx^2 of the points in the cube and the box
 #pragma unroll
@@ -551,9 +566,9 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
   float2 *sum_b = sum_a + 64;
   float2 *red_a = sum_b + 64;  // per-warp double-float partials
   float2 *red_b = red_a + kMaxWarps;
-  cur += sizeof(float2) * (2 * kMaxWarps + 128);
+  cur += sizeof(float2) * (2 * kMaxWarps + 128);  // (16-byte multiples so far: alpha is read as float4)
   float *alpha = reinterpret_cast<float *>(cur);
-  cur += sizeof(float) * maxi * NLM;
+  cur += sizeof(float4) * maxi * kPart;
   // PAIR: the two CTAs' gathered c per (slot, lm), [rank][slot * NLM + lm] (each CTA writes
   // its row into both), the per-warp partials of the projector part of a_k and the two
   // CTAs' capacity flags
@@ -582,11 +597,13 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
   int *scratch = list_scratch_bytes(maxi, nw) <= 4 * ncu ? reinterpret_cast<int *>(U)
                                                          : reinterpret_cast<int *>(part_s + p.part_cap);
 
-  // this CTA's slice of global scratch: T of the units beyond the tensor memory and all unit words
-  // (both [batch][lane]), partial sums
+  // this CTA's slice of global scratch: T and words of the units beyond the tensor memory
+  // ([batch][lane]), partial sums, the items' runs
   float4 *gT = reinterpret_cast<float4 *>(proj_scratch + (size_t)blockIdx.x * p.proj_bytes_per_cta);
-  unsigned *gword = reinterpret_cast<unsigned *>(gT + (size_t)p.list_batches * 32 * kRun * NCH);
-  float4 *part_g = reinterpret_cast<float4 *>(gword + (size_t)p.list_batches * 32);
+  float4 *gmeta = gT + (size_t)p.list_batches * 32 * kRun * NCH;
+  float4 *part_g = gmeta + (size_t)p.list_batches * 32;
+  float4 *grun = part_g + (size_t)p.part_total * kPart;
+  const float4 *qtables = reinterpret_cast<const float4 *>(tables);
 
   float4 *P4 = reinterpret_cast<float4 *>(P);
   float4 *U4 = reinterpret_cast<float4 *>(U);
@@ -636,39 +653,64 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
     const int K = (int)(node / ((long long)p.Nx * p.Ny));
     const int Xs = I - p.nhx, Ys = J - p.nhy, Zs = K - p.nhz;
 
-    // ---- per-node image list and slots (warp 0); others clear P ----
-    if (warp == 0) {
-      int count = 0;
-      for (int base = 0; base < p.n_images; base += 32) {
-        const int i = base + lane;
-        bool ok = false;
-        if (i < p.n_images) {
-          const int4 b = *reinterpret_cast<const int4 *>(&images[i]);
-          const TypeDesc &td = p.types[b.w];
-          ok = b.x <= Xs + nx - 1 && b.x + td.fx - 1 >= Xs && b.y <= Ys + ny - 1 &&
-               b.y + td.fy - 1 >= Ys && b.z <= Zs + nz - 1 && b.z + td.fz - 1 >= Zs;
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, ok);
-        const int pos = count + __popc(m & ((1u << lane) - 1u));
-        if (ok && pos < maxi) img[pos] = i;
-        count += __popc(m);
+    // ---- images that meet the cube, in order; every warp looks at its share.  P cleared ----
+    const int share = (p.n_images + 32 * nw - 1) / (32 * nw) * 32;
+    const int i0 = warp * share, i1 = min(p.n_images, i0 + share);
+    auto meets = [&](int i) {
+      if (i >= i1) return false;
+      const int4 b = *reinterpret_cast<const int4 *>(&images[i]);
+      const TypeDesc &td = p.types[b.w];
+      return b.x <= Xs + nx - 1 && b.x + td.fx - 1 >= Xs && b.y <= Ys + ny - 1 &&
+             b.y + td.fy - 1 >= Ys && b.z <= Zs + nz - 1 && b.z + td.fz - 1 >= Zs;
+    };
+    {
+      int found = 0;
+      for (int base = i0; base < i1; base += 32)
+        found += __popc(__ballot_sync(0xffffffffu, meets(base + lane)));
+      if (lane == 0) wunits[warp] = found;
+    }
+    for (int e = threadIdx.x; e < (ncp >> 2); e += blockDim.x) P4[e] = zero4;
+    __syncthreads();
+    {
+      int at = 0, count = 0;
+      for (int w = 0; w < nw; w++) {
+        at += w < warp ? wunits[w] : 0;
+        count += wunits[w];
       }
-      __syncwarp();
-      const int n = min(count, maxi);
+      for (int base = i0; base < i1; base += 32) {
+        const bool ok = meets(base + lane);
+        const unsigned m = __ballot_sync(0xffffffffu, ok);
+        const int pos = at + __popc(m & ((1u << lane) - 1u));
+        if (ok && pos < maxi) img[pos] = base + lane;
+        at += __popc(m);
+      }
+      if (threadIdx.x == 0) {
+        cnt[0] = min(count, maxi);
+        cnt[2] = count > maxi;
+        cnt[5] = 0;
+      }
+    }
+    __syncthreads();
+    const int n_img = cnt[0];
+    if (warp == 0) {  // their rows, and the slots (images are sorted by atom)
       int slots = 0;
-      for (int base = 0; base < n; base += 32) {
+      for (int base = 0; base < n_img; base += 32) {
         const int k = base + lane;
         bool start = false;
         ImageMeta m{};
-        if (k < n) {
+        if (k < n_img) {
           m = images[img[k]];
           start = (k == 0) || images[img[k - 1]].atom != m.atom;
         }
         const unsigned starts = __ballot_sync(0xffffffffu, start);
         const int g = slots + __popc(starts & ((1u << lane) - 1u)) + (start ? 0 : -1);
-        if (k < n) {
+        if (k < n_img) {
+          const TypeDesc &td = p.types[m.type];
+          const int shift = (m.bx - Xs) & 3;  // which copy of the table has the cube's quads aligned
           rows[k] = ImgRow{(float)(m.bx - Xs), (float)(m.by - Ys), (float)(m.bz - Zs - zo0), (float)m.ox,
-                           (float)m.oy,        (float)m.oz,        m.type,                   g};
+                           (float)m.oy, (float)m.oz,
+                           (int)(m.tab_base + (long long)shift * __popc(td.chan_mask) * quad_table_channel(td)),
+                           m.type | (g << 4)};
           if (start) {
             slot_type[g] = m.type;
             slot_first[g] = k;
@@ -677,67 +719,112 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
         slots += __popc(starts);
       }
       if (lane == 0) {
-        slot_first[slots] = n;
-        cnt[0] = n;
+        slot_first[slots] = n_img;
         cnt[1] = slots;
-        cnt[2] = count > maxi;
-        cnt[5] = 0;
       }
-    } else {
-      for (int e = threadIdx.x - 32; e < (ncp >> 2); e += blockDim.x - 32) P4[e] = zero4;
     }
     __syncthreads();
-    const int n_img = cnt[0], n_slot = cnt[1];
+    const int n_slot = cnt[1];
+
+    // ---- runs of every item (thread t: item t), kept in the scratch slice; units per (image, warp)
+    // and per item.  The warp's lanes share the images whose boxes meet the bounds of its columns ----
+    int *hist = scratch, *order = scratch + kSortKeys * nw, *kw = order + 32 * nw;
+    int *item_units = kw + maxi * nw;
+    int2 *runs = reinterpret_cast<int2 *>(grun) + threadIdx.x;  // run i: + i * blockDim.x
+    int units = 0;
+    {
+      const bool mine = threadIdx.x < n_item;
+      const ListItem it(mine ? threadIdx.x : 0, ncol, nlc, nq, nzo);
+      const int row = it.column / nq;
+      const int r0 = __reduce_min_sync(0xffffffffu, mine ? row : ny), r1 = __reduce_max_sync(0xffffffffu, mine ? row : -1);
+      const int z0 = __reduce_min_sync(0xffffffffu, mine ? it.zb : nzo), z1 = __reduce_max_sync(0xffffffffu, mine ? it.ze : 0);
+      int n_run = 0;
+      for (int base = 0; base < n_img; base += 32) {
+        const int k = base + lane;
+        bool near = false;
+        if (k < n_img) {
+          const ImgRow g = load_row(rows + k);
+          const TypeDesc &td = p.types[g.type()];
+          near = (int)g.by <= r1 && (int)g.by + td.fy > r0 && (int)g.bz < z1 && (int)g.bz + td.fz > z0;
+        }
+        int total = 0;  // of image k
+        for (unsigned todo = __ballot_sync(0xffffffffu, near); todo; todo &= todo - 1) {
+          const int src = __ffs(todo) - 1;
+          const ListRun r = mine ? it.run(p, rows + base + src, nx, ihz) : ListRun{0, 0};
+          const int n = r.units(), t = __reduce_add_sync(0xffffffffu, n);
+          if (lane == src) total = t;
+          if (n) {
+            runs[(size_t)blockDim.x * n_run++] = make_int2((base + src) | (r.a << 10) | (r.b << 17), 0);
+            units += n;
+          }
+        }
+        if (k < n_img) kw[k * nw + warp] = total;
+      }
+      if (mine) item_units[threadIdx.x] = units | (n_run << 16);
+      const int most = __reduce_max_sync(0xffffffffu, units);
+      if (lane == 0) atomicMax(cnt + 5, most);
+    }
+    __syncthreads();
 
     // ---- items dealt to the threads by their number of units, the most first ----
-    int *hist = scratch, *order = scratch + kSortKeys * nw, *kw = order + 32 * nw;
-    int units = 0;
-    if (threadIdx.x < n_item) {
-      const ListItem it(threadIdx.x, ncol, nlc, nq, nzo);
-      for (int k = 0; k < n_img; k++) units += it.run(p, rows + k, nx, ihz).units();
-    }
-    const int most = __reduce_max_sync(0xffffffffu, units);
-    if (lane == 0) atomicMax(cnt + 5, most);
-    __syncthreads();
-    {
-      int shift = 0;
-      while ((cnt[5] >> shift) >= kSortKeys) shift++;
-      // key kSortKeys - 1 - units (threads without an item last); every warp's count per key
-      const int key = threadIdx.x < n_item ? kSortKeys - 1 - (units >> shift) : kSortKeys - 1;
-      unsigned mine = 0;
-      for (int q = 0; q < kSortKeys; q += 32) {
-        int c = 0;
-        for (int v = 0; v < 32; v++) {
-          const unsigned m = __ballot_sync(0xffffffffu, key == q + v);
-          if (key == q + v) mine = m;
-          if (lane == v) c = __popc(m);
-        }
-        hist[(q + lane) * nw + warp] = c;
+    int shift = 0;
+    while ((cnt[5] >> shift) >= kSortKeys) shift++;
+    // key kSortKeys - 1 - units (threads without an item last); every warp's count per key
+    const int key = threadIdx.x < n_item ? kSortKeys - 1 - (units >> shift) : kSortKeys - 1;
+    unsigned same = 0;
+    for (int q = kSortKeys - 32 - (((cnt[5] >> shift) >> 5) << 5); q < kSortKeys; q += 32) {
+      int c = 0;
+      for (int v = 0; v < 32; v++) {
+        const unsigned m = __ballot_sync(0xffffffffu, key == q + v);
+        if (key == q + v) same = m;
+        if (lane == v) c = __popc(m);
       }
-      __syncthreads();
-      if (warp == 0) warp_exclusive_scan(hist, kSortKeys * nw);
-      __syncthreads();
-      order[hist[key * nw + warp] + __popc(mine & ((1u << lane) - 1u))] = threadIdx.x;
+      hist[(q + lane) * nw + warp] = c;
+    }
+    const int key0 = kSortKeys - 32 - (((cnt[5] >> shift) >> 5) << 5);
+    __syncthreads();
+    if (warp == 0) {
+      warp_exclusive_scan(hist + key0 * nw, (kSortKeys - key0) * nw);
+    } else if (warp == 1) {  // the places of the partial sums: by image, warp, lane
+      const int total = warp_exclusive_scan(kw, n_img * nw);
+      for (int g = lane; g < n_slot; g += 32) slot_base[g] = kw[slot_first[g] * nw];
+      if (lane == 0) slot_base[n_slot] = total;
+    }
+    __syncthreads();
+    order[hist[key * nw + warp] + __popc(same & ((1u << lane) - 1u))] = threadIdx.x;
+    {  // place of every run's first partial sum
+      int i = 0;
+      int2 r = units ? runs[0] : make_int2(1023, 0);
+      for (int base = 0; base < n_img; base += 32) {
+        const int k = base + lane;
+        const int next = k + 1 < n_img || warp + 1 < nw ? (k < n_img ? kw[k * nw + warp + 1] : 0) : slot_base[n_slot];
+        unsigned todo = __ballot_sync(0xffffffffu, k < n_img && next != kw[k * nw + warp]);
+        for (; todo; todo &= todo - 1) {
+          const int q = base + __ffs(todo) - 1;
+          const bool on = (r.x & 1023) == q;
+          const int n = on ? ListRun{(r.x >> 10) & 127, r.x >> 17}.units() : 0;
+          int incl = n;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+          }
+          if (on) {
+            runs[(size_t)blockDim.x * i].y = kw[q * nw + warp] + incl - n;
+            i++;
+            r = i < (item_units[threadIdx.x] >> 16) ? runs[(size_t)blockDim.x * i] : make_int2(1023, 0);
+          }
+        }
+      }
     }
     __syncthreads();
     const int my = order[threadIdx.x];
     const bool has_item = my < n_item;
     const ListItem item(has_item ? my : 0, ncol, nlc, nq, nzo);
-    units = 0;
-    for (int k = 0; k < n_img; k++) {  // units per image of every warp
-      const int u = has_item ? item.run(p, rows + k, nx, ihz).units() : 0;
-      units += u;
-      const int t = __reduce_add_sync(0xffffffffu, u);
-      if (lane == 0) kw[k * nw + warp] = t;
-    }
+    units = has_item ? item_units[my] & 0xffff : 0;
     const int w_units = __reduce_max_sync(0xffffffffu, units);
     if (lane == 0) wunits[warp] = w_units;
     __syncthreads();
-    if (warp == 0) {
-      const int total = warp_exclusive_scan(kw, n_img * nw);
-      for (int g = lane; g < n_slot; g += 32) slot_base[g] = kw[slot_first[g] * nw];
-      if (lane == 0) slot_base[n_slot] = total;
-    }
     // batches (units of a warp's 32 lanes) before this warp's, and units before it in its quarter
     int batch0 = 0, batches = 0, quarter0 = 0;
     for (int w = 0; w < nw; w++) {
@@ -748,7 +835,6 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
       }
       batches += u;
     }
-    __syncthreads();
     const int n_part = slot_base[n_slot];
     bool overflow = cnt[2] || batches > p.list_batches || n_part > p.part_total;
     if constexpr (PAIR) {  // both CTAs take the capacity branch together
@@ -760,7 +846,7 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
       overflow = xflag[0] || xflag[1];
     } else {
       // the next node, read by every thread after this node's last barrier (the previous
-      // value was read before the barrier above)
+      // value was read before the barriers above)
       if (threadIdx.x == 0) cnt[3] = atomicAdd(status + 1, 1);
     }
     if (overflow) {  // capacity exceeded: report, NaN coefficients
@@ -775,101 +861,93 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
     float4 *part = n_part * kPart <= p.part_cap ? part_s : part_g;
     const int tm_units = max(0, min(w_units, list_units_per_quarter(NCH) - quarter0));
     const unsigned tmT = tquarter + (unsigned)(quarter0 * kTCols);
-    const unsigned tmW = tquarter + (unsigned)(kListColumns - kListHeads + quarter0);
+    const unsigned tmM = tquarter + (unsigned)(list_units_per_quarter(NCH) * kTCols + quarter0 * 4);
     float4 *wT = gT + (size_t)batch0 * 32 * kRun * NCH + lane;  // of unit u: + ((u * NCH + c) * kRun + k) * 32
-    unsigned *wword = gword + (size_t)batch0 * 32 + lane;       // of unit u: + u * 32
+    float4 *wmeta = gmeta + (size_t)batch0 * 32 + lane;         // of unit u: + u * 32
 
-    // ---- the units' words, then their T ----
+    // ---- the units: word, coordinates and T ----
     {
-      int u = 0;
-      for (int k = 0; k < n_img; k++) {
-        const ListRun r = has_item ? item.run(p, rows + k, nx, ihz) : ListRun{0, 0};
-        const int n = r.units();
-        int incl = n;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int t = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= o) incl += t;
-        }
-        const int place = kw[k * nw + warp] + incl - n;
-        for (int j = 0; j < n; j++)
-          wword[32 * u++] = unit_word(k, min(r.a + kRun * j, item.top - kRun), place + j);
-      }
-      for (; u < w_units; u++) wword[32 * u] = unit_word(0, item.zb, 0);
-    }
-    __syncwarp();
-    {
-      int prev = -1, covered = 0;  // planes of the image's run that the units before this one cover
+      const int2 *mine = reinterpret_cast<const int2 *>(grun) + item.index;
+      const bool k1 = (int)item.x + 1 < nx, k2 = (int)item.x + 2 < nx, k3 = (int)item.x + 3 < nx;
+      const int xq = (int)item.x >> 2;
+      int left = 0, a = 0, b = 0, place = 0, cmask = 0, plane = 0;
+      const float4 *tq = qtables;  // the column's quad of plane 0 of the box, channel 0
+      long long chan = 0;
+      ImgRow g{};
+      int i = 0;
       for (int u = 0; u < w_units; u++) {
-        const unsigned w = wword[32 * u];
-        const int k = (int)(w & 1023), z0 = (int)((w >> 10) & 63);
         float4 T[NCH][kRun];
+        float4 meta = make_float4(__uint_as_float(unit_word(0, item.zb, 0)), 0.f, 0.f, 0.f);
 #pragma unroll
         for (int c = 0; c < NCH; c++)
 #pragma unroll
-          for (int i = 0; i < kRun; i++) T[c][i] = zero4;
+          for (int q = 0; q < kRun; q++) T[c][q] = zero4;
         if (u < units) {
-          const ListRun r = item.run(p, rows + k, nx, ihz);
-          if (k != prev) covered = r.a;
-          prev = k;
-          const ImgRow g = load_row(rows + k);
-          const TypeDesc &td = p.types[g.type];
-          const int fx = td.fx, lx = (int)(item.x - g.bx), ly = (int)(item.y - g.by);
-          const float *tab = tables + images[img[k]].tab_base + (ly * fx + lx);
-          const int fxy = fx * td.fy, fvol = fxy * td.fz;
-          const float dx = fmaf(p.hxf, item.x - g.bx, g.ox), dy = fmaf(p.hyf, item.y - g.by, g.oy);
-#pragma unroll
-          for (int i = 0; i < kRun; i++) {
-            const int z = z0 + i, lz = z - (int)g.bz;
-            const float dz = fmaf(p.hzf, float(z) - g.bz, g.oz), r2yz = fmaf(dy, dy, dz * dz);
-            const bool inz = z >= covered && z < r.b;
-            float v[NCH][4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-              const float x = fmaf(p.hxf, float(q), dx);
-              const bool in = inz && lx + q >= 0 && lx + q < fx && (int)item.x + q < nx &&
-                              fmaf(x, x, r2yz) <= td.support_r2_f32;
-              int c = 0, ch = 0;
-#pragma unroll
-              for (int l = 0; l < 4; l++) {
-                if (!(MASK & (1 << l))) continue;
-                const bool have = td.chan_mask & (1 << l);
-                v[c][q] = in && have ? tab[lz * fxy + ch * fvol + q] : 0.f;
-                ch += have ? 1 : 0;
-                c++;
-              }
-            }
-#pragma unroll
-            for (int c = 0; c < NCH; c++) T[c][i] = make_float4(v[c][0], v[c][1], v[c][2], v[c][3]);
+          if (left == 0) {  // the item's next image
+            const int2 r = mine[(size_t)blockDim.x * i++];
+            const ListRun run{(r.x >> 10) & 127, r.x >> 17};
+            a = run.a;
+            b = run.b;
+            left = run.units();
+            place = r.y;
+            g = load_row(rows + (r.x & 1023));
+            const TypeDesc &td = p.types[g.type()];
+            cmask = td.chan_mask;
+            plane = quad_table_row(td) * td.fy;
+            chan = quad_table_channel(td);
+            tq = qtables + (g.tab + ((int)item.y - (int)g.by) * quad_table_row(td) + xq - ((int)g.bx >> 2));
           }
-          covered = z0 + kRun;
+          const int z0 = min(a, item.top - kRun);
+          meta = make_float4(__uint_as_float(unit_word(g.slot(), z0, place)), fmaf(p.hxf, item.x - g.bx, g.ox),
+                             fmaf(p.hyf, item.y - g.by, g.oy), fmaf(p.hzf, float(z0) - g.bz, g.oz));
+          const float4 *tz = tq + (z0 - (int)g.bz) * plane;
+          int c = 0, ch = 0;
+#pragma unroll
+          for (int l = 0; l < 4; l++) {
+            if (!(MASK & (1 << l))) continue;
+            const bool have = cmask & (1 << l);
+#pragma unroll
+            for (int q = 0; q < kRun; q++) {  // planes [a, b) of the unit's
+              float4 t = ldg_quad_if(have && z0 + q >= a && z0 + q < b, tz + ch * chan + q * plane);
+              t.y = k1 ? t.y : 0.f;
+              t.z = k2 ? t.z : 0.f;
+              t.w = k3 ? t.w : 0.f;
+              T[c][q] = t;
+            }
+            ch += have ? 1 : 0;
+            c++;
+          }
+          a = z0 + kRun;
+          place++;
+          left--;
         }
         __syncwarp();
         if (u < tm_units) {
 #pragma unroll
           for (int c = 0; c < NCH; c++) tmem_st16(tmT + (unsigned)(u * kTCols + 16 * c), T[c]);
-          tmem_st1(tmW + (unsigned)u, w);
+          tmem_st4(tmM + (unsigned)(4 * u), meta);
         } else {
 #pragma unroll
           for (int c = 0; c < NCH; c++)
 #pragma unroll
-            for (int i = 0; i < kRun; i++) wT[((u * NCH + c) * kRun + i) * 32] = T[c][i];
+            for (int q = 0; q < kRun; q++) wT[((u * NCH + c) * kRun + q) * 32] = T[c][q];
+          wmeta[32 * u] = meta;
         }
       }
       tmem_wait_st();
     }
-    auto load_unit = [&](int u, float4 (&T)[NCH][kRun], unsigned &w) {
+    auto load_unit = [&](int u, float4 (&T)[NCH][kRun], float4 &meta) {
       if (u < tm_units) {
 #pragma unroll
         for (int c = 0; c < NCH; c++) tmem_ld16(tmT + (unsigned)(u * kTCols + 16 * c), T[c]);
-        tmem_ld1(tmW + (unsigned)u, w);
-        tmem_wait_ld(T, w);
+        tmem_ld4(tmM + (unsigned)(4 * u), meta);
+        tmem_wait_ld(T, meta);
       } else {
-        w = wword[32 * u];
+        meta = wmeta[32 * u];
 #pragma unroll
         for (int c = 0; c < NCH; c++)
 #pragma unroll
-          for (int i = 0; i < kRun; i++) T[c][i] = wT[((u * NCH + c) * kRun + i) * 32];
+          for (int q = 0; q < kRun; q++) T[c][q] = wT[((u * NCH + c) * kRun + q) * 32];
       }
     };
     // the item's column in P (owned planes) and U
@@ -899,18 +977,15 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
 
       // ---- phase 1: projector gather  ||  pass A ----
       for (int u = 0; u < w_units; u++) {
-        float4 T[NCH][kRun];
-        unsigned w;
-        load_unit(u, T, w);
-        const ImgRow g = load_row(rows + (w & 1023u));
-        const int z0 = (int)((w >> 10) & 63u);
-        unsigned a = itemP + (unsigned)(z0 * PB);
+        float4 T[NCH][kRun], meta;
+        load_unit(u, T, meta);
+        const unsigned w = __float_as_uint(meta.x);
+        unsigned a = itemP + (unsigned)((int)((w >> 10) & 63u) * PB);
         float4 v[kRun];
 #pragma unroll
         for (int i = 0; i < kRun; i++, a += (unsigned)PB) v[i] = lds_quad(a);
         float c[NLM];
-        Chi::gather(p, T, v, fmaf(p.hxf, item.x - g.bx, g.ox), fmaf(p.hyf, item.y - g.by, g.oy),
-                    fmaf(p.hzf, float(z0) - g.bz, g.oz), c);
+        Chi::gather(p, T, v, meta.y, meta.z, meta.w, c);
         if (u < units) {
           float4 *dst = part + (size_t)(w >> 16) * kPart;
 #pragma unroll
@@ -1088,7 +1163,7 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
             const int l = p.rank_l[r];
             const float gl = (td.chan_mask & (1 << l)) ? float(td.gamma[l]) : 0.f;
             const float al = gl * cr_sum;
-            alpha[sl * NLM + r] = al * sc * Chi::norm(r);
+            alpha[sl * 4 * kPart + r] = al * sc * Chi::norm(r);
             ka.add(al * cr_sum);
           }
         });
@@ -1111,7 +1186,7 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
           const int l = p.rank_l[r];
           const float gl = (td.chan_mask & (1 << l)) ? float(td.gamma[l]) : 0.f;
           const float cv = cx[e] + cx[maxi * NLM + e];
-          alpha[e] = gl * cv * sc * Chi::norm(r);
+          alpha[sl * 4 * kPart + r] = gl * cv * sc * Chi::norm(r);
           kn.add(gl * cv * cv);
         }
         const DF np = df_warp_sum(df_of(kn));
@@ -1119,20 +1194,24 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
         __syncthreads();
       }
       for (int u = 0; u < w_units; u++) {
-        float4 T[NCH][kRun];
-        unsigned w;
-        load_unit(u, T, w);
-        const ImgRow g = load_row(rows + (w & 1023u));
-        const int z0 = (int)((w >> 10) & 63u);
+        float4 T[NCH][kRun], meta;
+        load_unit(u, T, meta);
+        const unsigned w = __float_as_uint(meta.x);
+        const float4 *al = reinterpret_cast<const float4 *>(alpha) + (w & 1023u) * kPart;
         float q[NLM];
 #pragma unroll
-        for (int s = 0; s < NLM; s++) q[s] = alpha[g.slot * NLM + s];
-        const unsigned a = itemU + (unsigned)(z0 * PB);
+        for (int i = 0; i < kPart; i++) {
+          const float4 t = al[i];
+          q[4 * i] = t.x;
+          if (4 * i + 1 < NLM) q[4 * i + 1] = t.y;
+          if (4 * i + 2 < NLM) q[4 * i + 2] = t.z;
+          if (4 * i + 3 < NLM) q[4 * i + 3] = t.w;
+        }
+        const unsigned a = itemU + (unsigned)((int)((w >> 10) & 63u) * PB);
         float4 v[kRun];
 #pragma unroll
         for (int i = 0; i < kRun; i++) v[i] = lds_quad(a + (unsigned)(i * PB));
-        Chi::scatter(p, T, v, fmaf(p.hxf, item.x - g.bx, g.ox), fmaf(p.hyf, item.y - g.by, g.oy),
-                     fmaf(p.hzf, float(z0) - g.bz, g.oz), q);
+        Chi::scatter(p, T, v, meta.y, meta.z, meta.w, q);
 #pragma unroll
         for (int i = 0; i < kRun; i++) sts_quad_if(u < units, a + (unsigned)(i * PB), v[i]);
       }

@@ -70,6 +70,15 @@ int lanczos_quad_list_chunks(int columns, int planes, int threads);
 size_t lanczos_quad_unit_bytes(const LanczosParams &p);
 size_t lanczos_quad_list_bytes(const LanczosParams &p);
 void lanczos_quad_place_partials(LanczosParams &p, int smem_optin);
+// kLayoutQuad: the radial tables as aligned quads (lanczos_quad.cuh), built from the plain FP32 ones.
+struct QuadTable {
+  long long src, dst;  // floats into the plain tables, float4 into the quad tables
+  int type;
+  float ox, oy, oz;    // box point 0 relative to the atom
+};
+long long quad_table_float4(const TypeDesc &td);  // of one table, all shifts and channels
+cudaError_t launch_quad_tables(const LanczosParams &p, const QuadTable *tabs, int n, const float *src,
+                               void *dst, cudaStream_t s);
 // kLayoutPair: clusters of two CTAs that fit on the device at once (0 if none)
 int lanczos_quad_pair_clusters(const LanczosParams &p, int block, size_t smem);
 
