@@ -8,11 +8,20 @@
 //   rho_i = (2/dV) sum_q w_iq f,  E_band = 2 sum w lambda f,
 //   -TS = (2/beta) sum w [f ln f + (1-f) ln(1-f)].
 //
-// One cooperative persistent launch runs every bisection step: each CTA reduces its slice
-// into one partial per step, a bounded grid barrier publishes the partials, and every CTA
-// sums them in the same fixed order, so all CTAs take the same branch and the result does
-// not depend on scheduling.  The barrier spins a bounded number of times and then reports
-// kStatusTimeout instead of waiting forever.
+// One cooperative persistent launch runs the whole search: each CTA reduces its slice into
+// partials, a bounded grid barrier publishes them, and every CTA sums them in the same fixed
+// order, so all CTAs take the same branch and the result does not depend on scheduling.  The
+// barrier spins a bounded number of times and then reports kStatusTimeout instead of waiting
+// forever.
+//
+// The bisection's midpoints are the same as ever, but few of them are evaluated: N_e grows with lf
+// (weights are not negative; checked, else every midpoint is evaluated), so a midpoint outside a
+// known interval [xl, xr] with N_e(xl) <= n_electrons < N_e(xr) needs no sum.  The interval comes from
+// three levels per pass in FP32, taken as known only where the sum is off by more than its error,
+// and from Newton steps in FP64.  FP64 exponentials are what a pass costs (2 lanes of FP64 per SM and
+// cycle), so the FP64 passes run over the entries whose occupation can differ from 0 and 1 inside
+// the interval, gathered in shared memory once; the others are a constant.
+//   Before: about 45 passes of FP64 exponentials over all entries, 14.6 ms for 132651 x 40.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -80,8 +89,49 @@ __device__ bool grid_barrier(unsigned *bar, int *status, int *flag_smem, long lo
   return *flag_smem != 0;
 }
 
+// Occupation 1 / (1 + exp(x)), x = beta (lam - lf), without the exponential where it rounds to 1 (x
+// below -37.5: exp(x) < 2^-54) or underflows to 0 (x above 745.2).
 __device__ __forceinline__ double fermi_dirac(double beta, double lam, double lf) {
-  return 1.0 / (1.0 + exp(beta * (lam - lf)));
+  const double x = beta * (lam - lf);
+  if (x < -37.5) return 1.0;
+  if (x > 745.2) return 0.0;
+  return 1.0 / (1.0 + exp(x));
+}
+
+// The float nearest towards zero, by the bits (conversions run at the FP64 rate); for |v| below 2^-126
+// zero, above 2^127 infinity.
+__device__ __forceinline__ float truncate_f32(double v) {
+  const int hi = __double2hiint(v), mag = hi & 0x7fffffff;
+  const int bits = (int)(((unsigned)(mag - (896 << 20)) << 3) | ((unsigned)__double2loint(v) >> 29));
+  const int r = mag < (897 << 20) ? 0 : mag >= (1150 << 20) ? 0x7f800000 : bits;
+  return __int_as_float(r | (hi & 0x80000000));
+}
+
+// In units of 1/beta: entries this far above a level count as empty in the gathered sums (their
+// occupation is below 2e-20, under half an ulp of any sum that holds a single state), and this far
+// below as full (exactly 1 in FP64).
+constexpr double kFermiAbove = 45.5, kFermiBelow = 37.5;
+constexpr int kFermiLevels = 3;    // levels per FP32 pass
+constexpr int kFermiRows = 2 * kFermiLevels + 2;  // scratch rows: partials of two passes, bracket
+constexpr int kFermiEntries = 4096;  // entries of a CTA's slice gathered in shared memory
+constexpr size_t kFermiSmem = sizeof(double) * 2 * kFermiEntries;
+
+// Totals of up to N partials per CTA (rows scratch + j * G), the same order in every CTA.
+template <int N>
+__device__ void grid_totals(const double *rows, int G, double *bcast, double (&t)[N]) {
+  if (threadIdx.x < 32) {
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+      double v = 0.0;
+      for (int i = threadIdx.x; i < G; i += 32) v += __ldcg(rows + (long long)j * G + i);
+      v = warp_sum_d(v);
+      if (threadIdx.x == 0) bcast[j] = v;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < N; j++) t[j] = bcast[j];
+  __syncthreads();
 }
 
 __global__ void __launch_bounds__(kFermiBlock)
@@ -90,34 +140,43 @@ __global__ void __launch_bounds__(kFermiBlock)
                  double tol, int maxit, double *__restrict__ rho, double *__restrict__ out,
                  double *__restrict__ scratch, unsigned *__restrict__ bar,
                  int *__restrict__ status, long long spin_limit, int skip_block) {
+  extern __shared__ double gathered[];  // [2][kFermiEntries]: lambda, w of the open entries
   __shared__ double red[kFermiBlock / 32];
   // fault injection of the timeout self-test: one CTA leaves before its first arrival, so
   // every other CTA's first barrier wait runs out
   if ((int)blockIdx.x == skip_block) return;
-  __shared__ double bcast[2];
-  __shared__ int flag;
+  __shared__ double bcast[kFermiLevels];
+  __shared__ int flag, n_open_s;
   const int G = gridDim.x;
   const long long n = n_nodes * nqp;
   const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long stride = (long long)G * blockDim.x;
+  double *bracket = scratch + (long long)(2 * kFermiLevels) * G;
+  int parity = 0;  // which half of the partial rows the next pass writes
 
-  // phase 0: bracket
+  // phase 0: bracket, and whether N_e is known to grow with the level
   double lo = 1e300, hi = -1e300;
+  bool plain = false;
   for (long long e = tid; e < n; e += stride) {
-    lo = fmin(lo, lambda[e]);
-    hi = fmax(hi, lambda[e]);
+    const double l = lambda[e];
+    lo = fmin(lo, l);
+    hi = fmax(hi, l);
+    // a weight below zero or not finite, a value not finite (exponent all ones)
+    const int wh = __double2hiint(w[e]), lh = __double2hiint(l);
+    plain = plain || (wh < 0 && (wh & 0x7fffffff)) || ((wh >> 20) & 2047) == 2047 || ((lh >> 20) & 2047) == 2047;
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
     hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
   }
+  plain = __syncthreads_or(plain);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = lo;
   __syncthreads();
   if (threadIdx.x == 0) {
     double m = red[0];
     for (int i = 1; i < kFermiBlock / 32; i++) m = fmin(m, red[i]);
-    scratch[blockIdx.x] = m;
+    bracket[blockIdx.x] = m;
   }
   __syncthreads();
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = hi;
@@ -125,40 +184,194 @@ __global__ void __launch_bounds__(kFermiBlock)
   if (threadIdx.x == 0) {
     double m = red[0];
     for (int i = 1; i < kFermiBlock / 32; i++) m = fmax(m, red[i]);
-    scratch[G + blockIdx.x] = m;
+    bracket[G + blockIdx.x] = m;
+    scratch[blockIdx.x] = plain ? 1.0 : 0.0;
   }
   if (!grid_barrier(bar, status, &flag, spin_limit)) return;
-  if (threadIdx.x == 0) {
-    double a = scratch[0], b = scratch[G];
-    for (int i = 1; i < G; i++) {
-      a = fmin(a, scratch[i]);
-      b = fmax(b, scratch[G + i]);
+  {
+    double a = 1e300, b = -1e300, q = 0.0;
+    if (threadIdx.x < 32) {
+      for (int i = threadIdx.x; i < G; i += 32) {
+        a = fmin(a, __ldcg(bracket + i));
+        b = fmax(b, __ldcg(bracket + G + i));
+        q += __ldcg(scratch + i);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        a = fmin(a, __shfl_xor_sync(0xffffffffu, a, o));
+        b = fmax(b, __shfl_xor_sync(0xffffffffu, b, o));
+        q += __shfl_xor_sync(0xffffffffu, q, o);
+      }
+      if (threadIdx.x == 0) {
+        bcast[0] = a - 1.0;
+        bcast[1] = b + 1.0;
+        bcast[2] = q;
+      }
     }
-    bcast[0] = a - 1.0;
-    bcast[1] = b + 1.0;
+    __syncthreads();
+    lo = bcast[0];
+    hi = bcast[1];
+    plain = bcast[2] != 0.0;
+    __syncthreads();
   }
+  parity = 1;  // the first half still holds the flags
+
+  // known interval: N_e(xl) <= n_electrons < N_e(xr)
+  double xl = -1e300, xr = 1e300;
+  const double inv_beta = 1.0 / beta;
+
+  // phase 1a: kFermiLevels levels per pass in FP32.  Of a level's sum S the rounding of lambda (1e-7
+  // of |lambda|, beta times that of the exponent) and of the float sums stay below err S.
+  if (!plain) {
+    double cl = lo, cr = hi;
+    const float bf = (float)beta;
+    const double span = fmax(fabs(lo), fabs(hi));
+    const double err = 1e-4 + 4e-7 * beta * span;
+    for (int pass = 0; pass < 24 && cr - cl > 0.25 * inv_beta && err < 0.25; pass++) {
+      float lev[kFermiLevels], c[kFermiLevels];
+#pragma unroll
+      for (int j = 0; j < kFermiLevels; j++) {
+        lev[j] = truncate_f32(cl + (cr - cl) * ((j + 1) / (double)(kFermiLevels + 1)));
+        c[j] = 0.f;
+      }
+      for (long long e = tid; e < n; e += stride) {
+        const float l = truncate_f32(lambda[e]), we = truncate_f32(w[e]);
+#pragma unroll
+        for (int j = 0; j < kFermiLevels; j++)
+          c[j] += we * __fdividef(1.f, 1.f + __expf(fminf(bf * (l - lev[j]), 80.f)));
+      }
+      double *rows = scratch + (long long)parity * kFermiLevels * G, t[kFermiLevels];
+      parity ^= 1;
+#pragma unroll
+      for (int j = 0; j < kFermiLevels; j++) {
+        const double v = block_sum_d(2.0 * (double)c[j], red);
+        if (threadIdx.x == 0) rows[(long long)j * G + blockIdx.x] = v;
+      }
+      if (!grid_barrier(bar, status, &flag, spin_limit)) return;
+      grid_totals(rows, G, bcast, t);
+      bool moved = false;
+#pragma unroll
+      for (int j = 0; j < kFermiLevels; j++) {
+        const double m = (double)lev[j], slack = err * fmax(t[j], n_electrons);
+        if (t[j] + slack < n_electrons && m > cl) {
+          cl = m;
+          moved = true;
+        }
+        if (t[j] - slack > n_electrons && m < cr) {
+          cr = m;
+          moved = true;
+        }
+      }
+      if (!moved || !(cl < cr)) break;
+    }
+    if (cl < cr) {
+      if (cl > lo) xl = cl;
+      if (cr < hi) xr = cr;
+    }
+  }
+
+  // phase 1b: the entries that are neither full nor empty for every level left; `full` their sum
+  const double open_lo = fmax(xl, lo) - kFermiBelow * inv_beta, open_hi = fmin(xr, hi) + kFermiAbove * inv_beta;
+  double full = 0.0;
+  bool in_smem = !plain;
+  if (threadIdx.x == 0) n_open_s = 0;
   __syncthreads();
-  lo = bcast[0];
-  hi = bcast[1];
+  if (in_smem) {
+    for (long long base = tid - threadIdx.x; base < n; base += stride) {
+      const long long e = base + threadIdx.x;
+      bool open = false;
+      double l = 0.0;
+      if (e < n) {
+        l = lambda[e];
+        open = l >= open_lo && l <= open_hi;
+        if (l < open_lo) full += 2.0 * w[e];
+      }
+      // places by warp: one warp after another in a fixed order
+      const unsigned m = __ballot_sync(0xffffffffu, open);
+      const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+      __shared__ int first[kFermiBlock / 32 + 1];
+      if (lane == 0) first[warp] = __popc(m);
+      __syncthreads();
+      int at = n_open_s, all = 0;
+      for (int i = 0; i < kFermiBlock / 32; i++) {
+        at += i < warp ? first[i] : 0;
+        all += first[i];
+      }
+      at += __popc(m & ((1u << lane) - 1u));
+      if (open && at < kFermiEntries) {
+        gathered[at] = l;
+        gathered[kFermiEntries + at] = w[e];
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) n_open_s += all;
+      __syncthreads();
+      if (n_open_s > kFermiEntries) break;  // uniform: this CTA sums over its whole slice instead
+    }
+    in_smem = n_open_s <= kFermiEntries;
+  }
+  const int n_open = n_open_s;
+
+  // N_e and its derivative at x, summed over all CTAs.  False if the barrier gave up.
+  auto evaluate = [&](double x, double &ne, double &dne) {
+    double c = 0.0, d = 0.0;
+    if (in_smem) {
+      c = full;
+      for (int i = threadIdx.x; i < n_open; i += kFermiBlock) {
+        const double f = fermi_dirac(beta, gathered[i], x), we = 2.0 * gathered[kFermiEntries + i];
+        c += we * f;
+        d += we * f * (1.0 - f);
+      }
+    } else {
+      for (long long e = tid; e < n; e += stride) {
+        const double f = fermi_dirac(beta, lambda[e], x), we = 2.0 * w[e];
+        c += we * f;
+        d += we * f * (1.0 - f);
+      }
+    }
+    c = block_sum_d(c, red);
+    d = block_sum_d(d, red);
+    double *rows = scratch + (long long)parity * kFermiLevels * G, t[2];
+    parity ^= 1;
+    if (threadIdx.x == 0) {
+      rows[blockIdx.x] = c;
+      rows[G + blockIdx.x] = d;
+    }
+    if (!grid_barrier(bar, status, &flag, spin_limit)) return false;
+    grid_totals(rows, G, bcast, t);
+    ne = t[0];
+    dne = beta * t[1];
+    return true;
+  };
+
+  // phase 1c: Newton steps from inside the interval, every evaluation narrows it; once a step is
+  // within tol, one more evaluation just across the root
+  if (!plain && xl > -1e300 && xr < 1e300) {
+    const double near = fmax(0.25 * tol, 4e-16 * fmax(fabs(xl), fabs(xr)));
+    double x = 0.5 * (xl + xr);
+    for (int k = 0; k < 12 && xr - xl > 2.0 * near; k++) {
+      double ne, dne;
+      if (!evaluate(x, ne, dne)) return;
+      const bool above = ne > n_electrons;
+      if (above) xr = x;
+      else xl = x;
+      double next = x - (ne - n_electrons) / dne;
+      if (fabs(next - x) <= near) next = above ? next - near : next + near;  // the other side
+      if (!(next > xl && next < xr)) next = 0.5 * (xl + xr);
+      x = next;
+    }
+  }
 
   // phase 1: bisection on the electron count
   int it;
   for (it = 0; it < maxit; it++) {
     const double mid = 0.5 * (lo + hi);
-    double c = 0.0;
-    for (long long e = tid; e < n; e += stride) c += 2.0 * w[e] * fermi_dirac(beta, lambda[e], mid);
-    c = block_sum_d(c, red);
-    if (threadIdx.x == 0) scratch[(2 + it) * (long long)G + blockIdx.x] = c;
-    if (!grid_barrier(bar, status, &flag, spin_limit)) return;
-    if (threadIdx.x == 0) {
-      double ne = 0.0;
-      for (int i = 0; i < G; i++) ne += scratch[(2 + it) * (long long)G + i];
-      bcast[0] = ne;
+    bool above = mid >= xr;
+    if (!above && mid > xl) {
+      double ne, dne;
+      if (!evaluate(mid, ne, dne)) return;
+      above = ne > n_electrons;
     }
-    __syncthreads();
-    const double ne = bcast[0];
-    __syncthreads();
-    if (ne > n_electrons) hi = mid;
+    if (above) hi = mid;
     else lo = mid;
     if (hi - lo < tol) break;
   }
@@ -170,9 +383,11 @@ __global__ void __launch_bounds__(kFermiBlock)
     double r = 0.0;
     for (int q = 0; q < nqp; q++) {
       const long long e = node * nqp + q;
-      const double f = fermi_dirac(beta, lambda[e], lf);
+      const double l = lambda[e], x = beta * (l - lf);
+      if (x > 745.2) continue;  // empty
+      const double f = fermi_dirac(beta, l, lf);
       r += w[e] * f;
-      eb += 2.0 * w[e] * lambda[e] * f;
+      eb += 2.0 * w[e] * l * f;
       double s = 0.0;
       if (f > 0.0 && f < 1.0) s = f * log(f) + (1.0 - f) * log(1.0 - f);
       ent += 2.0 * w[e] * s;
@@ -181,22 +396,20 @@ __global__ void __launch_bounds__(kFermiBlock)
   }
   eb = block_sum_d(eb, red);
   ent = block_sum_d(ent, red);
-  const long long rowE = (2 + (long long)maxit) * G, rowS = rowE + G;
+  double *rows = scratch + (long long)parity * kFermiLevels * G, t[2];
   if (threadIdx.x == 0) {
-    scratch[rowE + blockIdx.x] = eb;
-    scratch[rowS + blockIdx.x] = ent;
+    rows[blockIdx.x] = eb;
+    rows[G + blockIdx.x] = ent;
   }
   if (!grid_barrier(bar, status, &flag, spin_limit)) return;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    double E = 0.0, S = 0.0;
-    for (int i = 0; i < G; i++) {
-      E += scratch[rowE + i];
-      S += scratch[rowS + i];
+  if (blockIdx.x == 0) {
+    grid_totals(rows, G, bcast, t);
+    if (threadIdx.x == 0) {
+      out[0] = lf;
+      out[1] = t[0];
+      out[2] = t[1] / beta;
+      out[3] = (double)it;
     }
-    out[0] = lf;
-    out[1] = E;
-    out[2] = S / beta;
-    out[3] = (double)it;
   }
 }
 
@@ -309,7 +522,9 @@ cudaError_t launch_electron_count(const double *lambda, const double *w, long lo
 // The message of sq_fermi_density_energy_noalloc failures, reported by sq_last_error_string.
 void set_noalloc_error(const std::string &msg);
 
-size_t fermi_scratch_doubles(int grid, int maxit) { return (size_t)grid * (maxit + 4); }
+size_t fermi_scratch_doubles(int grid, int maxit) {
+  return (size_t)grid * std::max(maxit + 4, kFermiRows);
+}
 
 namespace {
 cudaError_t launch_fermi_impl(const double *lambda, const double *w, long long n_nodes, int nqp,
@@ -323,8 +538,10 @@ cudaError_t launch_fermi_impl(const double *lambda, const double *w, long long n
                   (void *)&beta,   (void *)&n_electrons, (void *)&dV, (void *)&tol,
                   (void *)&maxit,  (void *)&rho, (void *)&out,     (void *)&scratch,
                   (void *)&barrier, (void *)&status, (void *)&spin_limit, (void *)&skip_block};
+  e = cudaFuncSetAttribute(fermi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFermiSmem);
+  if (e != cudaSuccess) return e;
   return cudaLaunchCooperativeKernel((const void *)fermi_kernel, dim3(grid), dim3(kFermiBlock),
-                                     args, 0, s);
+                                     args, kFermiSmem, s);
 }
 }  // namespace
 
@@ -433,7 +650,9 @@ extern "C" sq_status sq_fermi_density_energy_noalloc(const double *d_lambda,
   NoallocScratch *scr = reinterpret_cast<NoallocScratch *>(ptr);
   int sms = 0, per_sm = 0;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess ||
-      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fermi_kernel, kFermiBlock, 0)) !=
+      (e = cudaFuncSetAttribute(fermi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFermiSmem)) !=
+          cudaSuccess ||
+      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fermi_kernel, kFermiBlock, kFermiSmem)) !=
           cudaSuccess) {
     set_noalloc_error(std::string("device query: ") + cudaGetErrorString(e));
     return SQ_CUDA_ERROR;
