@@ -59,9 +59,8 @@ typedef struct sq_options {
    * split-pass kernel (SQ_BAD_INPUT where it does not apply). */
   int kernel;
   /* Split-pass kernel tile: z-ranges per cube row in the z pass and y-ranges per plane in the
-   * y pass (threads = ceil(nx/4) * max(ny,nz) * tile); 0 automatic (the engine's autotuner
-   * times the candidates on the first call and keeps the fastest).  The two-CTA form runs
-   * one tile and needs 0. */
+   * y pass (threads = ceil(nx/4) * max(ny,nz) * tile); 0 automatic (by the cube's size,
+   * with the number of CTAs that share an SM).  The two-CTA form runs one tile and needs 0. */
   int tile;
 } sq_options;
 

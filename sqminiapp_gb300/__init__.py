@@ -53,7 +53,7 @@ class LSDFT:
     the FP32 corrected operator's projector-list records (0 automatic, 1 full chi_lm, 2
     compact radial values; sq_options.list_format); kernel the FP32 Lanczos kernel (0
     automatic, 1 single-pass, 2 split-pass) and tile the split-pass kernel's z-/y-ranges per
-    row (0: timed on the first call).
+    row (0: by the cube size).
     """
 
     def __init__(self, deck_dir, name, faithful=False, precision=32, device=0, list_format=0,

@@ -359,31 +359,44 @@ void plan_engine(sq_handle *h, int smem_optin, int l2_bytes) {
     sq::LanczosParams q = p;
     q.layout = sq::kLayoutQuad;
     q.pitch = q.upitch = 4 * ((p.nx + 3) / 4);
-    q.zchunks = h->opt.tile > 0 ? h->opt.tile : 2;
-    const int threads = sq::lanczos_quad_threads(q);
-    // list bounds for every tile that may run
-    q.part_total = q.list_batches = q.part_cap = 0;
-    bool words = true;
-    for (int tile = h->opt.tile > 0 ? h->opt.tile : 1; tile <= std::max(4, h->opt.tile); tile++) {
-      sq::LanczosParams t = q;
-      t.zchunks = tile;
-      if (wide || sq::lanczos_quad_threads(t) > sq::kQuadMaxThreads) break;
-      words = quad_list_bounds(s, d, q, sq::lanczos_quad_block(t)) && words;
-      if (h->opt.tile > 0) break;
-    }
     // The lists of all CTAs, were none of them in tensor memory, must stay in L2 (what exceeds it is
     // streamed from there): units of whole boxes, 0.47 of which the spheres fill (27^3 cube).
     auto list_bytes = [&](const sq::LanczosParams &l) {
       return (double)h->num_sms * 0.47 * l.part_total * (double)sq::lanczos_quad_unit_bytes(l);
     };
-    if (!wide && threads <= sq::kQuadMaxThreads && words &&
-        sq::lanczos_quad_smem_bytes(q) <= (size_t)smem_optin &&
-        (h->opt.list_format == 1 || list_bytes(q) <= 0.75 * (double)l2_bytes)) {
-      p = q;
+    // Tile (plane / row ranges per thread walk) and CTAs per SM: the most threads in the stencil
+    // passes, a walk of L planes counted as L / (L + 5) for the 12 it loads first and the 16-warp
+    // kernels, with 128 registers, as 0.85.  Measured with every tile (ms per 3648 nodes, 20 steps; the
+    // chosen one first): 13^3 2.20 (tile 2, 3 CTAs), 2.40, 2.74; 17^3 3.50 (2, 2 CTAs), 4.10, 4.20; 19^3
+    // 3.97 (2, 2 CTAs), 4.61; 21^3 5.42 (3), 5.78, 6.06; 23^3 6.39 (3), 7.15; 27^3 9.74 (2), 13.20.
+    double best = 0.0;
+    sq::LanczosParams chosen = q;
+    for (int tile = h->opt.tile > 0 ? h->opt.tile : 1; !wide && tile <= std::max(4, h->opt.tile); tile++) {
+      sq::LanczosParams t = q;
+      t.zchunks = tile;
+      const int threads = sq::lanczos_quad_threads(t), block = sq::lanczos_quad_block(t);
+      if (threads > sq::kQuadMaxThreads) break;
+      t.part_total = t.list_batches = t.part_cap = 0;
+      const bool words = quad_list_bounds(s, d, t, block);
+      if (words && sq::lanczos_quad_smem_bytes(t) <= (size_t)smem_optin &&
+          (h->opt.list_format == 1 || list_bytes(t) <= 0.75 * (double)l2_bytes)) {
+        const int ctas = sq::lanczos_quad_place_partials(t, block, smem_optin);
+        const double walk = (double)((p.nz + tile - 1) / tile);
+        const double score = (double)ctas * (p.ny * (t.pitch / 4) * tile) * walk / (walk + 5.0) *
+                             (block > 384 ? 0.85 : 1.0);
+        if (score > best) {
+          best = score;
+          chosen = t;
+          h->quad_ctas = ctas;
+        }
+      }
+      if (h->opt.tile > 0) break;
+    }
+    if (best > 0.0) {
+      p = chosen;
       h->quad = true;
       h->u_smem = true;
-      h->block = sq::lanczos_quad_block(q);
-      sq::lanczos_quad_place_partials(p, smem_optin);
+      h->block = sq::lanczos_quad_block(p);
     } else if (h->opt.tile == 0 && p.nz >= 2 * sq::kStencilHalf + 2) {
       // the same kernel on a pair of CTAs per node, the cube split in z: each holds its half
       // of U and its half of P plus 6 halo planes; each streams its half of the list
@@ -391,8 +404,8 @@ void plan_engine(sq_handle *h, int smem_optin, int l2_bytes) {
       q.zsplit = (p.nz + 1) / 2;
       q.zchunks = 1;
       q.ychunks = 2;
-      q.part_total = q.list_batches = 0;
-      words = quad_list_bounds(s, d, q, sq::kPairThreads);
+      q.part_total = q.list_batches = q.part_cap = 0;
+      const bool words = quad_list_bounds(s, d, q, sq::kPairThreads);
       int pt = sq::lanczos_quad_threads(q);
       if (pt > sq::kPairThreads) {
         q.ychunks = 1;
@@ -406,8 +419,7 @@ void plan_engine(sq_handle *h, int smem_optin, int l2_bytes) {
         // all 12 warps of the register budget: the stencil passes use pt threads, the list
         // streams and the update all of them (fewer, longer warp ranges are slower)
         h->block = sq::kPairThreads;
-        sq::lanczos_quad_place_partials(p, smem_optin);
-        h->tuned = true;  // one tile
+        sq::lanczos_quad_place_partials(p, h->block, smem_optin);
       }
     }
   }
@@ -459,7 +471,8 @@ void plan_engine(sq_handle *h, int smem_optin, int l2_bytes) {
     throw std::invalid_argument("cube of " + std::to_string(p.nx) + "x" + std::to_string(p.ny) +
                                 "x" + std::to_string(p.nz) +
                                 " does not fit in shared memory at this precision");
-  h->grid = h->num_sms;
+  h->quad_ctas = h->quad && !(p.layout & sq::kLayoutPair) ? h->quad_ctas : 1;
+  h->grid = h->num_sms * h->quad_ctas;
   if (!h->quad) {  // projector records pack the P and U indices of a cube point into 16 bits each
     const long long pitch_rows = (p.layout & sq::kLayoutYGap) ? p.ny + sq::kStencilHalf : p.ny;
     const long long psize = (long long)sq::kStencilHalf * p.pitch + (long long)p.nz * pitch_rows * p.pitch;
@@ -629,46 +642,9 @@ sq_status run_device(sq_handle *h, const double *d_veff, double veff_const, long
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   ck(cudaStreamIsCapturing(s, &cap), "capture status");
   const bool timed = cap == cudaStreamCaptureStatusNone;  // no timing events inside a graph
-  if (h->quad && !h->tuned && h->opt.tile == 0 && timed && n >= 2LL * grid) {
-    // autotune the split-pass kernel's tile (z- / y-ranges per row / plane) on this call's
-    // first nodes, one node per CTA per candidate, and keep the fastest for the handle
-    cudaEvent_t t0, t1;
-    ck(cudaEventCreate(&t0), "event");
-    ck(cudaEventCreate(&t1), "event");
-    float best = 1e30f;
-    int best_tile = p.zchunks;
-    for (int tile = 1; tile <= 4; tile++) {
-      sq::LanczosParams q = p;
-      q.zchunks = tile;
-      q.node_end = nb + grid;
-      const int threads = sq::lanczos_quad_threads(q);
-      if (threads > sq::kQuadMaxThreads) break;
-      float ms = 0.f;
-      for (int rep = 0; rep < 2; rep++) {  // the first launch of a tile loads its code
-        ck(cudaEventRecord(t0, s), "event");
-        ck(sq::launch_lanczos(q, 32, false, true, grid, sq::lanczos_quad_block(q), h->smem, s,
-                              h->d_veff_ext,
-                              h->d_images, h->d_tables, h->d_u, h->d_proj, h->d_ab, h->d_status),
-           "lanczos (tile probe)");
-        ck(cudaEventRecord(t1, s), "event");
-        ck(cudaEventSynchronize(t1), "event");
-        ck(cudaEventElapsedTime(&ms, t0, t1), "event");
-      }
-      if (ms < best) {
-        best = ms;
-        best_tile = tile;
-      }
-    }
-    cudaEventDestroy(t0);
-    cudaEventDestroy(t1);
-    h->lp.zchunks = p.zchunks = best_tile;
-    h->block = sq::lanczos_quad_block(p);
-    h->info.kernel_threads = h->block;
-    h->tuned = true;
-  }
   if (timed) {
     update_node_cost(h);
-    h->cost_grid = grid;
+    h->cost_grid = grid_limit > 0 ? grid : std::max(1, grid / h->quad_ctas);  // SMs
     h->cost_nodes = n;
     ck(cudaEventRecord(h->ev[0], s), "event");
   }

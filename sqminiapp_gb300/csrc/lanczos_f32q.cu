@@ -69,13 +69,21 @@ size_t lanczos_quad_list_bytes(const LanczosParams &p) {
          sizeof(int2) * (size_t)p.max_img * kQuadMaxThreads;  // runs of every item
 }
 
-void lanczos_quad_place_partials(LanczosParams &p, int smem_optin) {
+int lanczos_quad_place_partials(LanczosParams &p, int block, int smem_optin) {
   // part_total counts whole boxes; the units of the spheres in them are about half (2161 of 4608 on
   // a 27^3 cube).  A node with more keeps its partial sums in the scratch slice.
   p.part_cap = 0;
-  const size_t room = ((size_t)smem_optin - lanczos_quad_smem_bytes(p)) / sizeof(float4);
-  const size_t want = partial_float4(p) * (size_t)(0.6 * p.part_total + 1);
-  p.part_cap = (int)std::min(room, want);
+  const size_t base = lanczos_quad_smem_bytes(p), reserved = 1024, sm = (size_t)smem_optin + reserved;
+  const size_t want = sizeof(float4) * partial_float4(p) * (size_t)(0.6 * p.part_total + 1);
+  // CTAs on an SM by shared memory (the partial sums included) and by registers: 12 warps of the
+  // 168-register kernels, one CTA of the others
+  int ctas = 1;
+  if (!(p.layout & kLayoutPair) && block <= 384)
+    ctas = std::max(1, std::min(std::min(4, 12 / (block / 32)), (int)(sm / (base + want + reserved))));
+  p.list_columns = ctas > 2 ? lq::kListColumns / 4 : lq::kListColumns / ctas;
+  const size_t room = sm / ctas - reserved - base;
+  p.part_cap = (int)(std::min(room, want) / sizeof(float4));
+  return ctas;
 }
 
 // ---- quad tables ----

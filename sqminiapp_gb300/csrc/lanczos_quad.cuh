@@ -242,10 +242,10 @@ __host__ __device__ constexpr int pair_u_planes(int nz, int zsplit) {
 // another, zero outside the support and the run.  A thread owns one column of quads over a range of
 // planes ("item") and its units, so no two threads ever meet on a quad.
 constexpr int kRun = 4;
-constexpr int kListColumns = 512;  // the whole tensor memory of an SM
+constexpr int kListColumns = 512;  // the whole tensor memory of an SM, shared by its CTAs
 // Units of a quarter (32 of the 128 lanes): T, the word and (x, y, z) relative to the atom.
-__host__ __device__ constexpr int list_units_per_quarter(int nch) {
-  return kListColumns / (4 * kRun * nch + 4);
+__host__ __device__ constexpr int list_units_per_quarter(int columns, int nch) {
+  return columns / (4 * kRun * nch + 4);
 }
 // Plane ranges per column: as many as the threads allow with at least kRun planes each.
 __host__ __device__ constexpr int list_chunks(int columns, int planes, int threads) {
@@ -616,7 +616,7 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
   const int PB = 16 * PS4, RB = 16 * nq;  // bytes of a plane and of a row
   // list items: column (quad xq of row y) and plane range [nzo c / nlc, nzo (c+1) / nlc) of the owned
   const int ncol = nq * ny, nlc = list_chunks(ncol, nzo, blockDim.x), n_item = ncol * nlc;
-  if (warp == 0) tc5::tmem_alloc(reinterpret_cast<uint32_t *>(cnt + 4), kListColumns);
+  if (warp == 0) tc5::tmem_alloc(reinterpret_cast<uint32_t *>(cnt + 4), (uint32_t)p.list_columns);
   __syncthreads();
   const float ihz = 1.f / p.hzf;
   const unsigned tquarter = (unsigned)cnt[4] + ((unsigned)(warp & 3) << 21);  // the warp's lanes
@@ -859,9 +859,9 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
       continue;
     }
     float4 *part = n_part * kPart <= p.part_cap ? part_s : part_g;
-    const int tm_units = max(0, min(w_units, list_units_per_quarter(NCH) - quarter0));
+    const int tm_units = max(0, min(w_units, list_units_per_quarter(p.list_columns, NCH) - quarter0));
     const unsigned tmT = tquarter + (unsigned)(quarter0 * kTCols);
-    const unsigned tmM = tquarter + (unsigned)(list_units_per_quarter(NCH) * kTCols + quarter0 * 4);
+    const unsigned tmM = tquarter + (unsigned)(list_units_per_quarter(p.list_columns, NCH) * kTCols + quarter0 * 4);
     float4 *wT = gT + (size_t)batch0 * 32 * kRun * NCH + lane;  // of unit u: + ((u * NCH + c) * kRun + k) * 32
     float4 *wmeta = gmeta + (size_t)batch0 * 32 + lane;         // of unit u: + u * 32
 
@@ -1316,7 +1316,7 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
   }
   // no CTA of a pair leaves while its peer may still read its shared memory
   if constexpr (PAIR) cooperative_groups::this_cluster().sync();
-  if (warp == 0) tc5::tmem_dealloc((unsigned)cnt[4], kListColumns);
+  if (warp == 0) tc5::tmem_dealloc((unsigned)cnt[4], (uint32_t)p.list_columns);
 }
 
 template <int MASK, int MAXT, bool ISO>

@@ -75,6 +75,7 @@ struct LanczosParams {
   // kLayoutQuad, per node at most: list units, batches of 32 of them; float4 of shared memory for
   // their partial sums
   int part_total, list_batches, part_cap;
+  int list_columns;        // kLayoutQuad: tensor-memory columns of a CTA
   long long proj_bytes_per_cta;
   long long node_begin, node_end;
   double hx, hy, hz;

@@ -64,12 +64,13 @@ int lanczos_quad_threads(const LanczosParams &p);
 // threads to launch a single-CTA split-pass kernel with (>= lanczos_quad_threads)
 int lanczos_quad_block(const LanczosParams &p);
 // The kernel's projector list: planes of a unit, plane ranges per column of quads, bytes of a unit and
-// of one CTA's slice of global scratch; and room in shared memory for the units' partial sums (part_cap).
+// of one CTA's slice of global scratch; and room in shared memory for the units' partial sums (part_cap)
+// with the CTAs that share an SM (returned) and their tensor-memory columns (list_columns).
 constexpr int kQuadListRun = 4;
 int lanczos_quad_list_chunks(int columns, int planes, int threads);
 size_t lanczos_quad_unit_bytes(const LanczosParams &p);
 size_t lanczos_quad_list_bytes(const LanczosParams &p);
-void lanczos_quad_place_partials(LanczosParams &p, int smem_optin);
+int lanczos_quad_place_partials(LanczosParams &p, int block, int smem_optin);
 // kLayoutQuad: the radial tables as aligned quads (lanczos_quad.cuh), built from the plain FP32 ones.
 struct QuadTable {
   long long src, dst;  // floats into the plain tables, float4 into the quad tables
