@@ -25,6 +25,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <random>
 #include <string>
 #include <vector>
@@ -168,7 +169,7 @@ __global__ void pack_features_kernel(const float *__restrict__ raw, long long n,
        e += (long long)gridDim.x * blockDim.x) {
     const long long row = e / kFeat;
     const int f = (int)(e % kFeat);
-    const float v = row < n ? (raw[e] - mean[f]) * inv_std[f] : 0.f;
+    const float v = row < n ? (mean ? (raw[e] - mean[f]) * inv_std[f] : raw[e]) : 0.f;
     const long long t = row / kTile;
     const uint32_t r = (uint32_t)(row % kTile);
     st_bf16(xa + t * kXTileBytes, tc5::tile_offset(r, f, kFeat), v);
@@ -628,18 +629,60 @@ struct sq_mlp {
   long long adam_step = 0;
   int partial_rows = 0;
   std::mt19937_64 rng{12345};
+  // buffers of sq_mlp_forward / sq_mlp_gradients (MlpWork)
+  std::mutex work_lock;
+  uint8_t *d_work = nullptr;
+  size_t work_cap = 0;
 
   ~sq_mlp() {
     for (float **p : {&d_params, &d_m, &d_v, &d_grad, &d_partial, &d_mean, &d_istd, &d_raw, &d_tgt_raw, &d_t,
                       &d_mask})
       dev_free(*p);
-    for (uint8_t **p : {&d_w1p, &d_w2p, &d_w2tp, &d_xa, &d_xt}) dev_free(*p);
+    for (uint8_t **p : {&d_w1p, &d_w2p, &d_w2tp, &d_xa, &d_xt, &d_work}) dev_free(*p);
     dev_free(d_status);
     dev_free(d_tiles);
   }
 };
 
 namespace {
+
+// Device buffers of one call, cut from one block that the network keeps between calls (allocating and
+// freeing them took 250 of 412 us for 39304 samples, a 10 MB copy among them 60).  A call that needs more
+// than kKeep gets a block of its own; calls on one network take turns.
+class MlpWork {
+ public:
+  MlpWork(sq_mlp *m, std::initializer_list<size_t> sizes) : lock_(m->work_lock) {
+    size_t total = 0;
+    for (size_t b : sizes) total += padded(b);
+    constexpr size_t kKeep = size_t(64) << 20;
+    if (total > kKeep) {
+      dev_alloc(&own_, total, "mlp work");
+      at_ = own_;
+      return;
+    }
+    if (total > m->work_cap) {
+      dev_free(m->d_work);
+      m->work_cap = 0;
+      dev_alloc(&m->d_work, total, "mlp work");
+      m->work_cap = total;
+    }
+    at_ = m->d_work;
+  }
+  ~MlpWork() { dev_free(own_); }
+  MlpWork(const MlpWork &) = delete;
+  MlpWork &operator=(const MlpWork &) = delete;
+  // the next buffer, in the order and of the sizes given to the constructor
+  template <typename T> T *take(size_t bytes) {
+    T *p = reinterpret_cast<T *>(at_);
+    at_ += padded(bytes);
+    return p;
+  }
+
+ private:
+  static size_t padded(size_t b) { return (b + 255) & ~size_t(255); }
+  std::lock_guard<std::mutex> lock_;
+  uint8_t *own_ = nullptr, *at_ = nullptr;
+};
 
 void mlp_alloc(sq_mlp *m) {
   ck(cudaSetDevice(m->device), "cudaSetDevice");
@@ -1025,24 +1068,22 @@ sq_status sq_mlp_gradients(sq_mlp *m, const float *x, const float *t, long n, do
     ck(cudaSetDevice(m->device), "cudaSetDevice");
     cudaStream_t s = 0;
     const long long nt = (n + kTile - 1) / kTile, np = nt * kTile;
-    DevBuf<float> x_d(sizeof(float) * (size_t)n * kFeat, "x"), t_d(sizeof(float) * n, "t"),
-        tp_d(sizeof(float) * np, "t"), mask_d(sizeof(float) * np, "mask"),
-        zero_d(sizeof(float) * kFeat, "zero"), one_d(sizeof(float) * kFeat, "one");
-    DevBuf<uint8_t> xa_d((size_t)nt * kXTileBytes, "xa"), xt_d((size_t)nt * kXTileBytes, "xt");
-    std::vector<float> z(kFeat, 0.f), o(kFeat, 1.f);
-    ck(cudaMemcpy(zero_d.get(), z.data(), sizeof(float) * kFeat, cudaMemcpyHostToDevice), "H2D");
-    ck(cudaMemcpy(one_d.get(), o.data(), sizeof(float) * kFeat, cudaMemcpyHostToDevice), "H2D");
-    ck(cudaMemcpy(x_d.get(), x, sizeof(float) * (size_t)n * kFeat, cudaMemcpyHostToDevice), "x H2D");
-    ck(cudaMemcpy(t_d.get(), t, sizeof(float) * n, cudaMemcpyHostToDevice), "t H2D");
-    pack_features_kernel<<<grid_of(np * kFeat), 256, 0, s>>>(x_d.get(), n, np, zero_d.get(), one_d.get(),
-                                                             xa_d.get(), xt_d.get());
-    pack_targets_kernel<<<grid_of(np), 256, 0, s>>>(t_d.get(), n, np, 0.f, 1.f, tp_d.get(), mask_d.get());
+    const size_t xb = sizeof(float) * (size_t)n * kFeat, tb = sizeof(float) * n, pb = sizeof(float) * np,
+                 ab = (size_t)nt * kXTileBytes;
+    MlpWork work(m, {xb, tb, pb, pb, ab, ab});
+    float *x_d = work.take<float>(xb), *t_d = work.take<float>(tb), *tp_d = work.take<float>(pb),
+          *mask_d = work.take<float>(pb);
+    uint8_t *xa_d = work.take<uint8_t>(ab), *xt_d = work.take<uint8_t>(ab);
+    ck(cudaMemcpyAsync(x_d, x, xb, cudaMemcpyHostToDevice, s), "x H2D");
+    ck(cudaMemcpyAsync(t_d, t, tb, cudaMemcpyHostToDevice, s), "t H2D");
+    pack_features_kernel<<<grid_of(np * kFeat), 256, 0, s>>>(x_d, n, np, nullptr, nullptr, xa_d, xt_d);
+    pack_targets_kernel<<<grid_of(np), 256, 0, s>>>(t_d, n, np, 0.f, 1.f, tp_d, mask_d);
     ck_launch("pack");
     // every tile once, one tile per CTA
     std::vector<int> tiles((size_t)nt);
     for (long long i = 0; i < nt; i++) tiles[i] = (int)i;
     pack_weights(m, s);
-    run_train_kernel(m, TileSet{xa_d.get(), xt_d.get(), tp_d.get(), mask_d.get()}, tiles, 1,
+    run_train_kernel(m, TileSet{xa_d, xt_d, tp_d, mask_d}, tiles, 1,
                      1.0f / (float)n, s);
     std::vector<float> g(kPartial);
     ck(cudaMemcpy(g.data(), m->d_grad, sizeof(float) * kPartial, cudaMemcpyDeviceToHost), "grad D2H");
@@ -1060,22 +1101,19 @@ sq_status sq_mlp_forward(sq_mlp *m, const float *x, long n, float *y) {
     ck(cudaSetDevice(m->device), "cudaSetDevice");
     cudaStream_t s = 0;
     const long long nt = (n + kTile - 1) / kTile, np = nt * kTile;
-    DevBuf<float> x_d(sizeof(float) * (size_t)n * kFeat, "x"), y_d(sizeof(float) * n, "y"),
-        zero_d(sizeof(float) * kFeat, "zero"), one_d(sizeof(float) * kFeat, "one");
-    DevBuf<uint8_t> xa_d((size_t)nt * kXTileBytes, "xa");
-    std::vector<float> z(kFeat, 0.f), o(kFeat, 1.f);
-    ck(cudaMemcpy(zero_d.get(), z.data(), sizeof(float) * kFeat, cudaMemcpyHostToDevice), "H2D");
-    ck(cudaMemcpy(one_d.get(), o.data(), sizeof(float) * kFeat, cudaMemcpyHostToDevice), "H2D");
-    ck(cudaMemcpy(x_d.get(), x, sizeof(float) * (size_t)n * kFeat, cudaMemcpyHostToDevice), "x H2D");
-    pack_features_kernel<<<grid_of(np * kFeat), 256, 0, s>>>(x_d.get(), n, np, zero_d.get(), one_d.get(),
-                                                             xa_d.get(), nullptr);
+    const size_t xb = sizeof(float) * (size_t)n * kFeat, yb = sizeof(float) * n, ab = (size_t)nt * kXTileBytes;
+    MlpWork work(m, {xb, yb, ab});
+    float *x_d = work.take<float>(xb), *y_d = work.take<float>(yb);
+    uint8_t *xa_d = work.take<uint8_t>(ab);
+    ck(cudaMemcpyAsync(x_d, x, xb, cudaMemcpyHostToDevice, s), "x H2D");
+    pack_features_kernel<<<grid_of(np * kFeat), 256, 0, s>>>(x_d, n, np, nullptr, nullptr, xa_d, nullptr);
     ck_launch("pack");
     pack_weights(m, s);
     const int grid = (int)std::min<long long>(nt, 2LL * m->num_sms);
-    mlp_forward_kernel<<<grid, 128, kFwdSmem, s>>>(xa_d.get(), nt, n, m->d_w1p, m->d_w2p, m->d_params,
-                                                   y_d.get(), m->d_status);
+    mlp_forward_kernel<<<grid, 128, kFwdSmem, s>>>(xa_d, nt, n, m->d_w1p, m->d_w2p, m->d_params, y_d,
+                                                   m->d_status);
     ck_launch("mlp forward");
-    ck(cudaMemcpy(y, y_d.get(), sizeof(float) * n, cudaMemcpyDeviceToHost), "y D2H");
+    ck(cudaMemcpy(y, y_d, yb, cudaMemcpyDeviceToHost), "y D2H");
     return mlp_status(m);
   });
 }
