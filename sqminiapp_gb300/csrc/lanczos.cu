@@ -11,8 +11,9 @@ namespace sq {
 
 namespace {
 
+// Veff (FP64: cdiag + Veff, as its stencil pass takes it) padded periodically by the cube half-width.
 template <typename T>
-__global__ void veff_extend_kernel(const double *__restrict__ veff, double vconst,
+__global__ void veff_extend_kernel(const double *__restrict__ veff, double vconst, double cdiag,
                                    T *__restrict__ ext, int Nx, int Ny, int Nz, int nhx, int nhy,
                                    int nhz, int EX, int EY, int EZ) {
   const long long total = (long long)EX * EY * EZ;
@@ -22,7 +23,8 @@ __global__ void veff_extend_kernel(const double *__restrict__ veff, double vcons
     const int gx = ((ex - nhx) % Nx + Nx) % Nx;
     const int gy = ((ey - nhy) % Ny + Ny) % Ny;
     const int gz = ((ez - nhz) % Nz + Nz) % Nz;
-    ext[e] = T(veff ? veff[((long long)gz * Ny + gy) * Nx + gx] : vconst);
+    const double v = veff ? veff[((long long)gz * Ny + gy) * Nx + gx] : vconst;
+    ext[e] = sizeof(T) == 8 ? T(cdiag + v) : T(v);
   }
 }
 
@@ -190,10 +192,10 @@ cudaError_t launch_veff_extend(const double *veff, double vconst, void *ext, int
   const int block = 256;
   const int grid = (int)std::min<long long>((total + block - 1) / block, 152LL * 16);
   if (precision == 32)
-    veff_extend_kernel<float><<<grid, block, 0, s>>>(veff, vconst, (float *)ext, p.Nx, p.Ny, p.Nz,
+    veff_extend_kernel<float><<<grid, block, 0, s>>>(veff, vconst, 0.0, (float *)ext, p.Nx, p.Ny, p.Nz,
                                                      p.nhx, p.nhy, p.nhz, p.EX, p.EY, p.EZ);
   else
-    veff_extend_kernel<double><<<grid, block, 0, s>>>(veff, vconst, (double *)ext, p.Nx, p.Ny,
+    veff_extend_kernel<double><<<grid, block, 0, s>>>(veff, vconst, p.cdiag, (double *)ext, p.Nx, p.Ny,
                                                       p.Nz, p.nhx, p.nhy, p.nhz, p.EX, p.EY, p.EZ);
   return cudaGetLastError();
 }

@@ -19,8 +19,11 @@
 // pair (x, x+1) from 64-bit shared loads, forming neighbour sums with Blackwell's packed
 // add.rn.f32x2, and walks z with a 13-plane register ring, so one output costs ~10 shared
 // loads.  Cubes wider than 32 points (WIDE) give each thread one (row, x pair) over all of
-// z instead, consecutive threads on consecutive pairs.  FP64 uses one warp per row with
-// scalar loads.
+// z instead, consecutive threads on consecutive pairs.  FP64 gives each lane one (x, y) column
+// over a z-range, 32 consecutive columns to a warp, with scalar loads: the FP64 pipe (2 lanes per
+// SM and cycle) bounds these passes, 84% busy, and a warp per row of 27 (21) points left 16% (34%)
+// of its lanes empty.  Against a warp per row, with cdiag folded into Veff and the scaling of h left to
+// the update: 27^3, 2001 nodes of 40 steps 234.3 -> 195.9 ms; 21^3 (the Mg1 deck) 57.8 -> 43.3 ms.
 // Nonlocal term: when a node starts, its projector matrix restricted to the cube (support
 // points only) is written once to a per-CTA list in global scratch: per point the packed
 // P/U indices and chi_lm (chi_lm = T_l(r) P_lm(x,y,z), from the per-atom radial tables and
@@ -84,6 +87,22 @@ template <typename T> __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
+}
+
+// Sums of four values over the warp: value s (this lane's, lane / 8), valid in every lane of its
+// eight.  The values are halved with the lanes first: 6 additions a lane instead of 20.
+template <typename T> __device__ __forceinline__ T warp_sum4(const T (&v)[4], int &s) {
+  const int lane = threadIdx.x & 31;
+  const bool h16 = lane & 16, h8 = lane & 8;
+  T a = h16 ? v[2] : v[0], b = h16 ? v[3] : v[1];
+  a += __shfl_xor_sync(0xffffffffu, h16 ? v[0] : v[2], 16);
+  b += __shfl_xor_sync(0xffffffffu, h16 ? v[1] : v[3], 16);
+  T c = h8 ? b : a;
+  c += __shfl_xor_sync(0xffffffffu, h8 ? a : b, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+  s = lane >> 3;
+  return c;
 }
 
 // Sum of one double per thread over the CTA (nw warps); red holds kMaxWarps+1 doubles.
@@ -290,6 +309,20 @@ __device__ __forceinline__ void decode(const ImgView<T> &v, int t, int &lx, int 
   ly = row - lz * v.ey;
 }
 
+// z-ranges (1..4) of the FP64 column items: the fewest plane steps of the busiest warp, a range
+// counted with 3 more for its first loads.
+__device__ __forceinline__ int columns_z_ranges(int groups, int nz, int nw) {
+  int best = 1, cost = 1 << 30;
+  for (int c = 1; c <= 4; c++) {
+    const int t = (groups * c + nw - 1) / nw * ((nz + c - 1) / c + 3);
+    if (t < cost) {
+      cost = t;
+      best = c;
+    }
+  }
+  return best;
+}
+
 template <typename T, bool FAITHFUL, bool U_SMEM, int MASK, int LAYOUT>
 __global__ void __launch_bounds__((LAYOUT & kLayoutWide) ? 32 * kWideWarpsF32 : 512, 1)
     lanczos_kernel(const __grid_constant__ LanczosParams p, const T *__restrict__ veff_ext,
@@ -366,11 +399,10 @@ __global__ void __launch_bounds__((LAYOUT & kLayoutWide) ? 32 * kWideWarpsF32 : 
   unsigned *ridx = reinterpret_cast<unsigned *>(
       reinterpret_cast<unsigned char *>(rec) + (size_t)p.proj_cap * sizeof(typename Rec::vec_t) * Rec::nvec);
 
-  const int x = lane;
-  const bool xin = x < nx;
-  const int xc = xin ? x : nx - 1;
-  const int y_begin = warp * p.rows_per_warp;
-  const int y_end = min(ny, y_begin + p.rows_per_warp);
+  // FP64 vector passes: items of 32 columns (x fastest) by a z-range, dealt to the warps in turn;
+  // as many z-ranges as even out the warps' shares (a range of zlen64 planes loads 12 more first)
+  const int ncol = nx * ny, ncg = (ncol + 31) >> 5;
+  const int nz64 = columns_z_ranges(ncg, nz, nw), zlen64 = (nz + nz64 - 1) / nz64;
   // FP32 vector passes: half-warp hw owns row py and a z-chunk [zb, ze); lane hl owns the x
   // pair (px, px+1) with px even.  pact = the pair has a cube point, phi = so does px+1.
   constexpr bool PAIRED = sizeof(T) == 4;
@@ -656,10 +688,16 @@ __global__ void __launch_bounds__((LAYOUT & kLayoutWide) ? 32 * kWideWarpsF32 : 
             }
           }
           const int sl = slot[k];
+          if constexpr (CSTRIDE == 4) {
+            int s;
+            const T r = warp_sum4(acc, s);
+            if ((lane & 7) == 0) atomicAdd(&cacc[sl * CSTRIDE + s], r);
+          } else {
 #pragma unroll
-          for (int s = 0; s < CSTRIDE; s++) {
-            const T r = warp_sum(acc[s]);
-            if (lane == 0) atomicAdd(&cacc[sl * CSTRIDE + s], r);
+            for (int s = 0; s < CSTRIDE; s++) {
+              const T r = warp_sum(acc[s]);
+              if (lane == 0) atomicAdd(&cacc[sl * CSTRIDE + s], r);
+            }
           }
           pos = kend;
           k++;
@@ -753,47 +791,48 @@ __global__ void __launch_bounds__((LAYOUT & kLayoutWide) ? 32 * kWideWarpsF32 : 
           pair_pass1(py, pxc, phi, zb, ze);
         }
       } else {
-        for (int y = y_begin; y < y_end; y++) {
-          const int rowP = OFF + y * pitch + xc;
-          const int rowU = y * upitch + xc;
-          const T *vrow = veff_ext + ((size_t)K * p.EY + (J + y)) * p.EX + (I + xc);
+        for (int item = warp; item < ncg * nz64; item += nw) {
+          const int zr = item / ncg, cg = item - zr * ncg;
+          const bool in = cg * 32 + lane < ncol;
+          const int col = min(cg * 32 + lane, ncol - 1), y = col / nx, x = col - y * nx;
+          const int zb64 = zr * zlen64, ze64 = min(nz, zb64 + zlen64);
+          const int rowP = OFF + y * pitch + x;
+          const T *vrow = veff_ext + ((size_t)K * p.EY + (J + y)) * p.EX + (I + x);
           const size_t VS = (size_t)p.EY * p.EX;
           T win[W];
   #pragma unroll
-          for (int q = -O; q < O; q++)
-            win[q + O + 1] = (q >= 0 && q < nz) ? P[rowP + min(max(q, 0), nz - 1) * PS] : T(0);
+          for (int q = -O; q < O; q++) {
+            const int zq = zb64 + q;
+            win[q + O + 1] = (zq >= 0 && zq < nz) ? P[rowP + min(max(zq, 0), nz - 1) * PS] : T(0);
+          }
   #pragma unroll 1
-          for (int z = 0; z < nz; z++) {
+          for (int z = zb64; z < ze64; z++) {
   #pragma unroll
             for (int t = 0; t < W - 1; t++) win[t] = win[t + 1];
             const int qn = z + O;
             win[W - 1] = (qn < nz) ? P[rowP + min(qn, nz - 1) * PS] : T(0);
-            const int i = rowP + z * PS;
+            const int i = rowP + z * PS, u = col + z * US;
+            const T uo = U[u];
             const T vc = win[O];
-            T h = (Coef<T>::diag(p) + vrow[z * VS]) * vc;
+            T h = vrow[z * VS] * vc;  // FP64: cdiag + Veff
   #pragma unroll
             for (int d = 1; d <= O; d++) {
               h += Coef<T>::z(p, d) * (win[O - d] + win[O + d]);
               if constexpr (XCLAMP) {  // no zero columns between rows: clamp, then drop
-                const T xm = P[xc - d >= 0 ? i - d : i];
-                const T xp = P[xc + d < nx ? i + d : i];
-                h += Coef<T>::x(p, d) * ((xc - d >= 0 ? xm : T(0)) + (xc + d < nx ? xp : T(0)));
+                const T xm = P[x - d >= 0 ? i - d : i];
+                const T xp = P[x + d < nx ? i + d : i];
+                h += Coef<T>::x(p, d) * ((x - d >= 0 ? xm : T(0)) + (x + d < nx ? xp : T(0)));
               } else {
                 h += Coef<T>::x(p, d) * (P[i - d] + P[i + d]);
               }
-              if constexpr (YPAD) {
-                h += Coef<T>::y(p, d) * (P[i - d * pitch] + P[i + d * pitch]);
-              } else {  // rows outside the cube are zero: clamp the index, then drop the value
-                const T ym = P[y - d >= 0 ? i - d * pitch : i];
-                const T yp = P[y + d < ny ? i + d * pitch : i];
-                h += Coef<T>::y(p, d) * ((y - d >= 0 ? ym : T(0)) + (y + d < ny ? yp : T(0)));
-              }
+              // rows outside the cube are zero: clamp the index, then drop the value
+              const T ym = P[y - d >= 0 ? i - d * pitch : i];
+              const T yp = P[y + d < ny ? i + d * pitch : i];
+              h += Coef<T>::y(p, d) * ((y - d >= 0 ? ym : T(0)) + (y + d < ny ? yp : T(0)));
             }
-            h *= inv;
-            if (xin) {
-              const int u = rowU + z * US;
-              a_acc += (vc * inv) * h;
-              U[u] = h - tbeta * U[u];
+            if (in) {
+              a_acc += vc * h;  // scaled by inv^2 below
+              U[u] = inv * h - tbeta * uo;
             }
           }
         }
@@ -879,6 +918,7 @@ __global__ void __launch_bounds__((LAYOUT & kLayoutWide) ? 32 * kWideWarpsF32 : 
           k++;
         }
       }
+      if constexpr (!PAIRED) a_acc *= inv * inv;
       const double a = block_sum((double)a_acc + a_part, red, nw);
 
       // ---- pass 2: w = U - a_k v_k, P <- w, U <- v_k, b_k = ||w|| ----
@@ -913,16 +953,18 @@ __global__ void __launch_bounds__((LAYOUT & kLayoutWide) ? 32 * kWideWarpsF32 : 
         } else if (pact) {
           pair_pass2(py, pxc, phi, zb, ze);
         }
-      } else if (xin) {
-        for (int y = y_begin; y < y_end; y++) {
-          const int rowP = OFF + y * pitch + x;
-          const int rowU = y * upitch + x;
-          for (int z = 0; z < nz; z++) {
+      } else {
+        for (int item = warp; item < ncg * nz64; item += nw) {
+          const int zr = item / ncg, cg = item - zr * ncg, col = cg * 32 + lane;
+          if (col >= ncol) continue;
+          const int y = col / nx, rowP = OFF + y * pitch + col - y * nx;
+          const int zb64 = zr * zlen64, ze64 = min(nz, zb64 + zlen64);
+          for (int z = zb64; z < ze64; z++) {
             const T pv = P[rowP + z * PS];
             const T vk = pv * inv;
-            const T w = U[rowU + z * US] - ta * vk;
+            const T w = U[col + z * US] - ta * vk;
             P[rowP + z * PS] = w;
-            U[rowU + z * US] = vk;
+            U[col + z * US] = vk;
             b_acc += w * w;
           }
         }
