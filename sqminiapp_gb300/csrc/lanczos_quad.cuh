@@ -120,18 +120,19 @@ __device__ __forceinline__ float4 lds_quad(unsigned a) {
                : "memory");
   return v;
 }
-__device__ __forceinline__ void lds_quad_if(bool on, unsigned a, float4 &v) {
+// at a + OFS, the offset in the instruction
+template <int OFS> __device__ __forceinline__ void lds_quad_if(bool on, unsigned a, float4 &v) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %5, 0;\n\t@p ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+      "{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %5, 0;\n\t@p ld.shared.v4.f32 {%0, %1, %2, %3}, [%4+%6];\n\t}"
       : "+f"(v.x), "+f"(v.y), "+f"(v.z), "+f"(v.w)
-      : "r"(a), "r"((int)on)
+      : "r"(a), "r"((int)on), "n"(OFS)
       : "memory");
 }
-__device__ __forceinline__ void lds_pair_if(bool on, unsigned a, float2 &v) {
+template <int OFS> __device__ __forceinline__ void lds_pair_if(bool on, unsigned a, float2 &v) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %3, 0;\n\t@p ld.shared.v2.f32 {%0, %1}, [%2];\n\t}"
+      "{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %3, 0;\n\t@p ld.shared.v2.f32 {%0, %1}, [%2+%4];\n\t}"
       : "+f"(v.x), "+f"(v.y)
-      : "r"(a), "r"((int)on)
+      : "r"(a), "r"((int)on), "n"(OFS)
       : "memory");
 }
 __device__ __forceinline__ void sts_quad_if(bool on, unsigned a, float4 v) {
@@ -505,25 +506,27 @@ __device__ __forceinline__ int warp_exclusive_scan(int *v, int n) {
   return __shfl_sync(0xffffffffu, incl, 31);
 }
 
-// Sum of N values over the warp; the total of value i goes to fn(i, total) in one lane.  N = 4 halves
-// the values with the lanes first (6 shuffles instead of 20).
-template <int N, typename FN> __device__ __forceinline__ void warp_totals(const float (&v)[N], FN &&fn) {
+// Sums of N values over each G lanes; the total of value i goes to fn(i, total) in one of them.  N = 4
+// halves the values with the lanes first (G = 32: 6 shuffles instead of 20).
+template <int G, int N, typename FN> __device__ __forceinline__ void group_totals(const float (&v)[N], FN &&fn) {
   const int lane = threadIdx.x & 31;
   if constexpr (N == 4) {
-    const bool h16 = lane & 16, h8 = lane & 8;
-    float a = h16 ? v[2] : v[0], b = h16 ? v[3] : v[1];
-    a += __shfl_xor_sync(0xffffffffu, h16 ? v[0] : v[2], 16);
-    b += __shfl_xor_sync(0xffffffffu, h16 ? v[1] : v[3], 16);
-    float c = h8 ? b : a;
-    c += __shfl_xor_sync(0xffffffffu, h8 ? a : b, 8);
+    const bool hi = lane & (G / 2), mid = lane & (G / 4);
+    float a = hi ? v[2] : v[0], b = hi ? v[3] : v[1];
+    a += __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[2], G / 2);
+    b += __shfl_xor_sync(0xffffffffu, hi ? v[1] : v[3], G / 2);
+    float c = mid ? b : a;
+    c += __shfl_xor_sync(0xffffffffu, mid ? a : b, G / 4);
 #pragma unroll
-    for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-    if ((lane & 7) == 0) fn(lane >> 3, c);
+    for (int o = G / 8; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    if ((lane & (G / 4 - 1)) == 0) fn((lane & (G - 1)) / (G / 4), c);
   } else {
 #pragma unroll
     for (int s = 0; s < N; s++) {
-      const float r = lk::warp_sum(v[s]);
-      if (lane == 0) fn(s, r);
+      float r = v[s];
+#pragma unroll
+      for (int o = G / 2; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+      if ((lane & (G - 1)) == 0) fn(s, r);
     }
   }
 }
@@ -965,7 +968,7 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
     const int sh = (4 - (I & 3)) & 3;
     const float4 *vq = reinterpret_cast<const float4 *>(veffq + (size_t)sh * p.vq_copy_stride) +
                        (size_t)((I + sh) >> 2);
-    const size_t VPS4 = (size_t)p.EY * (p.vq_row >> 2);  // plane stride in quads
+    const int VPS4 = p.EY * (p.vq_row >> 2);             // plane stride in quads
     const size_t VRS4 = (size_t)(p.vq_row >> 2);         // row stride in quads
 
     float sc = 1.f;          // s_k
@@ -1025,8 +1028,7 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
         if constexpr (kAhead) {
           nuo = lds_quad(aU);
           dv1 = __ldg(vrow);
-          dv2 = ldg_quad_if(1 < live, vrow + VPS4);
-          vrow += 2 * VPS4;
+          dv2 = __ldg(vrow + min(1, live - 1) * VPS4);
         }
         for (int i0 = 0; i0 < zlen; i0 += W) {
 #pragma unroll
@@ -1035,23 +1037,22 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
             if (i >= zlen) break;
             ring[s] = lds_quad(i < above ? aN : sZ);
 #define RING(dd) ring[(s + (dd) + O + 1) % W]
-            lds_pair_if(hm2, aP - 24u, xm2);
-            lds_quad_if(hm1, aP - 16u, xm1);
-            lds_quad_if(hp1, aP + 16u, xp1);
-            lds_pair_if(hp2, aP + 32u, xp2);
+            lds_pair_if<-24>(hm2, aP, xm2);
+            lds_quad_if<-16>(hm1, aP, xm1);
+            lds_quad_if<16>(hp1, aP, xp1);
+            lds_pair_if<32>(hp2, aP, xp2);
             const float4 c = RING(0);
             float4 dv, uo;
             if constexpr (kAhead) {
               dv = dv1;
               dv1 = dv2;
-              dv2 = ldg_quad_if(i + 2 < live, vrow);
+              dv2 = __ldg(vrow + min(i + 2, live - 1) * VPS4);
               uo = nuo;
-              lds_quad_if(i + 1 < live, aU + (unsigned)PB, nuo);
+              lds_quad_if<0>(i + 1 < live, aU + (unsigned)PB, nuo);
             } else {
-              dv = ldg_quad_if(i < live, vrow);
+              dv = __ldg(vrow + min(i, live - 1) * VPS4);
               uo = lds_quad(i < live ? aU : sZ);
             }
-            vrow += VPS4;
             float2 h01 = mul2(lo(dv), lo(c)), h23 = mul2(hi(dv), hi(c));
 #pragma unroll
             for (int d = 1; d <= O; d++) {
@@ -1114,7 +1115,7 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
             if (i >= ylen) break;
             const float4 uo = nuo;
             const float4 nring = lds_quad(i < above ? aN : sZ);
-            lds_quad_if(i + 1 < live, aU + (unsigned)RB, nuo);
+            lds_quad_if<0>(i + 1 < live, aU + (unsigned)RB, nuo);
 #define RING(dd) ring[(s + (dd) + O) % W]
             float2 h01 = mul2(cys[1], add2(lo(RING(-1)), lo(RING(1))));
             float2 h23 = mul2(cys[1], add2(hi(RING(-1)), hi(RING(1))));
@@ -1135,24 +1136,29 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
           }
         }
       }
-      // c of every slot, its units' partial sums in a fixed order, one warp per slot; alpha =
-      // Gamma_l s c (the harmonics' constants on both sides), <P, V_nl P> = sum Gamma_l c^2
-      for (int sl = warp; sl < n_slot; sl += nw) {
-        float c[NLM];
+      // c of every slot, its units' partial sums in a fixed order; alpha = Gamma_l s c (the harmonics'
+      // constants on both sides), <P, V_nl P> = sum Gamma_l c^2.  A warp per slot, or with more slots
+      // than warps eight lanes (4864 nodes: 32 atoms, 27^3 24.2 -> 23.2 ms; 4 atoms, 25^3 15.4 against
+      // 15.9 with a warp; the pair and the 16-warp kernels lose 2% with eight).
+      {
+        auto sum_slot = [&](int sl, int first, int step, float (&c)[NLM]) {
 #pragma unroll
-        for (int s = 0; s < NLM; s++) c[s] = 0.f;
-        for (int j = slot_base[sl] + lane; j < slot_base[sl + 1]; j += 32) {
+          for (int s = 0; s < NLM; s++) c[s] = 0.f;
+          const int end = sl < n_slot ? slot_base[sl + 1] : 0;
+#pragma unroll 4
+          for (int j = sl < n_slot ? slot_base[sl] + first : 0; j < end; j += step) {
 #pragma unroll
-          for (int i = 0; i < kPart; i++) {
-            const float4 t = part[(size_t)j * kPart + i];
-            c[4 * i] += t.x;
-            if (4 * i + 1 < NLM) c[4 * i + 1] += t.y;
-            if (4 * i + 2 < NLM) c[4 * i + 2] += t.z;
-            if (4 * i + 3 < NLM) c[4 * i + 3] += t.w;
+            for (int i = 0; i < kPart; i++) {
+              const float4 t = part[(size_t)j * kPart + i];
+              c[4 * i] += t.x;
+              if (4 * i + 1 < NLM) c[4 * i + 1] += t.y;
+              if (4 * i + 2 < NLM) c[4 * i + 2] += t.z;
+              if (4 * i + 3 < NLM) c[4 * i + 3] += t.w;
+            }
           }
-        }
-        __syncwarp();
-        warp_totals<NLM>(c, [&](int r, float total) {
+          __syncwarp();
+        };
+        auto finish = [&](int sl, int r, float total) {
           const float cr_sum = total * Chi::norm(r);
           if constexpr (PAIR) {  // this CTA's part of c, into both CTAs' row cr of cx
             float *x = cx + cr * maxi * NLM + sl * NLM + r;
@@ -1166,7 +1172,22 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
             alpha[sl * 4 * kPart + r] = al * sc * Chi::norm(r);
             ka.add(al * cr_sum);
           }
-        });
+        };
+        float c[NLM];
+        if (PAIR || MAXT > 384 || n_slot <= nw) {
+          for (int sl = warp; sl < n_slot; sl += nw) {
+            sum_slot(sl, lane, 32, c);
+            group_totals<32, NLM>(c, [&](int r, float total) { finish(sl, r, total); });
+          }
+        } else {
+          for (int s0 = warp * 4; s0 < n_slot; s0 += nw * 4) {
+            const int sl = s0 + (lane >> 3);
+            sum_slot(sl, lane & 7, 8, c);
+            group_totals<8, NLM>(c, [&](int r, float total) {
+              if (sl < n_slot) finish(sl, r, total);
+            });
+          }
+        }
       }
       {
         const DF ap = df_warp_sum(df_of(ka));
