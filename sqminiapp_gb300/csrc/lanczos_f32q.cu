@@ -37,7 +37,7 @@ size_t lanczos_quad_smem_bytes(const LanczosParams &p) {
   if (pair)  // both CTAs' c, an 8-byte alignment, projector a_k partials, capacity flags
     b += sizeof(float) * 2 * (size_t)p.max_img * nlm + 8 + sizeof(float) * 2 * lk::kMaxWarps +
          sizeof(int) * 4;
-  b += sizeof(int) * (4 * (size_t)p.max_img + 2 + 6 + lk::kMaxWarps);  // per-node lists
+  b += sizeof(int) * (4 * (size_t)p.max_img + 2 + 5 + lk::kMaxWarps);  // per-node lists
   b += 16 + sizeof(lq::ImgRow) * (size_t)p.max_img + sizeof(float4);   // image rows, a quad of zeros
   b += sizeof(float4) * (size_t)p.part_cap;
   const size_t scratch = lq::list_scratch_bytes(p.max_img, kQuadMaxThreads / 32);

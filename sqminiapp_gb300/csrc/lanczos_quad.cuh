@@ -209,13 +209,28 @@ __device__ __forceinline__ DF df_all_reduce(const float2 *red, int nw) {
   return df_warp_sum(DF{r.x, r.y});
 }
 
-// Floats per z-plane of P and U: ny rows of pitch, plus a pad that makes the plane stride
-// congruent to one row (4 * pitch/4 floats) modulo the 32 banks.  The y pass has nq = pitch/4
-// consecutive threads per plane and consecutive planes on consecutive thread groups, so its
-// float4 accesses then fall on consecutive banks across the whole warp (without the pad two
-// planes of a quarter-warp can share banks, e.g. 27 rows of 28 floats: offset 20 banks).
+// Floats per z-plane of P and U: ny rows of pitch, rounded up to all 32 banks, so that the bank of a
+// quad is that of its column (8 classes of columns) whatever its plane.  A quarter-warp reads or
+// writes its 8 quads at once if they are of 8 classes: the list's columns and pass B's are dealt to the
+// lanes that way (bank_slot).  Dealt by their number of units alone, over planes whose banks follow
+// on one another, a gather and a scatter of 27^3 took 7800 shared-memory wavefronts instead of 3450, of
+// 29^3 12000 instead of 4700: 39304 nodes of 27^3 and 40 steps 191.8 -> 179.7 ms, 17800 of 29^3 114.4 ->
+// 107.4 ms, 4864 of 33^3 on pairs 115.5 -> 110.7 ms (whole calls).
 __host__ __device__ constexpr int quad_plane_floats(int ny, int pitch) {
-  return ny * pitch + ((pitch - ny * pitch) % 32 + 32) % 32;
+  return (ny * pitch + 31) / 32 * 32;
+}
+// The thread of the rank-th column of bank class r: lane r of the rank-th group of 8; what a class has
+// beyond the groups goes where others have fewer.  size(r): columns of class r, their sum <= 8 groups.
+template <typename FN> __device__ __forceinline__ int bank_slot(int r, int rank, int groups, FN &&size) {
+  if (rank < groups) return 8 * rank + r;
+  int m = rank - groups;
+  for (int i = 0; i < r; i++) m += max(0, size(i) - groups);
+  for (int i = 0; i < 8; i++) {
+    const int n = size(i), free = max(0, groups - n);
+    if (m < free) return 8 * (n + m) + i;
+    m -= free;
+  }
+  return 0;  // not reached
 }
 
 // CTA pair (cube split in z at zsplit): CTA r owns planes [zo0, zo1) of P and U and keeps
@@ -257,11 +272,10 @@ __host__ __device__ constexpr int list_chunks(int columns, int planes, int threa
 __host__ __device__ constexpr int list_planes(int planes) {  // planes to allocate
   return planes < kRun ? kRun : planes;
 }
-constexpr int kSortKeys = 64;
-// Bytes of per-node scratch of the list build: a key histogram per warp, the items in order, unit
-// counts per (image, warp), units and runs per item.
+// Bytes of per-node scratch of the list build: the items in order, unit counts per (image, warp), units
+// and runs per item.
 __host__ __device__ constexpr int list_scratch_bytes(int max_img, int nw) {
-  return 4 * (kSortKeys * nw + 32 * nw + max_img * nw + 32 * nw);
+  return 4 * (32 * nw + max_img * nw + 32 * nw);
 }
 // The radial tables of this kernel hold whole quads: rows of the box's points behind `shift` zeros
 // (four copies, shift 0..3: the image's box start modulo 4 picks the one whose quads are the cube's),
@@ -590,8 +604,8 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
   int *slot_type = img + maxi;
   int *slot_first = slot_type + maxi;    // first image of every slot (images sorted by atom), n_img
   int *slot_base = slot_first + maxi + 1;  // first partial sums of every slot, their number
-  int *cnt = slot_base + maxi + 1;  // [0] images, [1] slots, [2] overflow, [3] next node, [4] TMEM, [5] most units
-  int *wunits = cnt + 6;            // units of every warp's longest lane
+  int *cnt = slot_base + maxi + 1;  // [0] images, [1] slots, [2] overflow, [3] next node, [4] TMEM
+  int *wunits = cnt + 5;            // units of every warp's longest lane
   ImgRow *rows = reinterpret_cast<ImgRow *>(
       (reinterpret_cast<uintptr_t>(wunits + kMaxWarps) + 15) & ~static_cast<uintptr_t>(15));
   float4 *zq = reinterpret_cast<float4 *>(rows + maxi);  // a quad of zeros
@@ -624,18 +638,41 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
   const float ihz = 1.f / p.hzf;
   const unsigned tquarter = (unsigned)cnt[4] + ((unsigned)(warp & 3) << 21);  // the warp's lanes
 
-  // thread -> quad of a row (pass A) / of a plane (pass B): nq consecutive threads own the
-  // quads of one row or plane, so consecutive threads touch consecutive 16-byte quads
+  // pass A: nq consecutive threads own the quads of a row, so consecutive threads touch consecutive
+  // quads.  Row yA, z-range [zbA, zeA) of the owned planes
   const int grp = threadIdx.x / nq, ql = threadIdx.x - grp * nq;
   const int nch = p.zchunks, nchB = PAIR ? p.ychunks : p.zchunks;
-  // pass A: row yA, z-range [zbA, zeA) of the owned planes
   const int yA = grp % ny, zcA = grp / ny;
   const int zlen = (nzo + nch - 1) / nch;
   const int zbA = zo0 + min(nzo, zcA * zlen), zeA = min(zo1, zbA + zlen);
   const bool actA = zcA < nch && zbA < zeA;
-  // pass B: owned plane zB, y-range [ybB, yeB)
-  const int zB = zo0 + grp % nzo, ycB = grp / nzo;
+  // pass B: quad qB of owned plane zB, y-range [ybB, yeB); the columns (y-range, plane, quad) dealt by
+  // the bank class of their first row, ranked by y-range, quad, plane
   const int ylen = (ny + nchB - 1) / nchB;
+  int colB;
+  {
+    auto of_class = [&](int c, int r) {  // quads of y-range c in class r
+      const int first = (r - c * ylen * nq) & 7;
+      return first < nq ? (nq - first + 7) >> 3 : 0;
+    };
+    scratch[threadIdx.x] = nchB * nzo * nq;
+    __syncthreads();
+    if ((int)threadIdx.x < nchB * nzo * nq) {
+      const int c = grp / nzo, r = (c * ylen * nq + ql) & 7;
+      int rank = (ql >> 3) * nzo + grp % nzo;
+      for (int i = 0; i < c; i++) rank += of_class(i, r) * nzo;
+      scratch[bank_slot(r, rank, (int)blockDim.x >> 3, [&](int i) {
+        int n = 0;
+        for (int k = 0; k < nchB; k++) n += of_class(k, i) * nzo;
+        return n;
+      })] = threadIdx.x;
+    }
+    __syncthreads();
+    colB = scratch[threadIdx.x];
+    __syncthreads();
+  }
+  const int grpB = colB / nq, qB = colB - grpB * nq;
+  const int zB = zo0 + grpB % nzo, ycB = grpB / nzo;
   const int ybB = min(ny, ycB * ylen), yeB = min(ny, ybB + ylen);
   const bool actB = ycB < nchB && ybB < yeB;
   // x neighbours of the quad inside the row; lanes of the last quad zero its pad points
@@ -690,7 +727,6 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
       if (threadIdx.x == 0) {
         cnt[0] = min(count, maxi);
         cnt[2] = count > maxi;
-        cnt[5] = 0;
       }
     }
     __syncthreads();
@@ -731,7 +767,7 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
 
     // ---- runs of every item (thread t: item t), kept in the scratch slice; units per (image, warp)
     // and per item.  The warp's lanes share the images whose boxes meet the bounds of its columns ----
-    int *hist = scratch, *order = scratch + kSortKeys * nw, *kw = order + 32 * nw;
+    int *order = scratch, *kw = order + 32 * nw;
     int *item_units = kw + maxi * nw;
     int2 *runs = reinterpret_cast<int2 *>(grun) + threadIdx.x;  // run i: + i * blockDim.x
     int units = 0;
@@ -763,41 +799,60 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
         }
         if (k < n_img) kw[k * nw + warp] = total;
       }
-      if (mine) item_units[threadIdx.x] = units | (n_run << 16);
-      const int most = __reduce_max_sync(0xffffffffu, units);
-      if (lane == 0) atomicMax(cnt + 5, most);
+      item_units[threadIdx.x] = units | (n_run << 16);
+      order[threadIdx.x] = n_item;
     }
     __syncthreads();
 
-    // ---- items dealt to the threads by their number of units, the most first ----
-    int shift = 0;
-    while ((cnt[5] >> shift) >= kSortKeys) shift++;
-    // key kSortKeys - 1 - units (threads without an item last); every warp's count per key
-    const int key = threadIdx.x < n_item ? kSortKeys - 1 - (units >> shift) : kSortKeys - 1;
-    unsigned same = 0;
-    for (int q = kSortKeys - 32 - (((cnt[5] >> shift) >> 5) << 5); q < kSortKeys; q += 32) {
-      int c = 0;
-      for (int v = 0; v < 32; v++) {
-        const unsigned m = __ballot_sync(0xffffffffu, key == q + v);
-        if (key == q + v) same = m;
-        if (lane == v) c = __popc(m);
+    // ---- items dealt to the lanes by their number of units, the most first: within their bank class;
+    // where the classes differ so much that this takes twice as many batches (units of a warp's 32
+    // lanes) as the units would fill, or more than there is room for, among all ----
+    const int own_units = units;
+    int my, w_units, n_part, batch0, batches, quarter0;  // batches before this warp's, units before it in its quarter
+    for (int step = 8;; step = 1) {
+      if ((int)threadIdx.x < n_item) {
+        const int r = step == 1 ? 0 : (int)threadIdx.x % ncol & 7;
+        int rank = 0;
+        for (int c = 0; c < n_item; c += ncol)
+#pragma unroll 4
+          for (int t = c + r; t < c + ncol; t += step) {
+            const int n = item_units[t] & 0xffff;
+            rank += n > own_units || (n == own_units && t < (int)threadIdx.x);
+          }
+        if (step == 8)
+          rank = bank_slot(r, rank, (int)blockDim.x >> 3, [&](int i) { return nlc * ((ncol - i + 7) >> 3); });
+        order[rank] = threadIdx.x;
       }
-      hist[(q + lane) * nw + warp] = c;
+      if (warp == 0 && step == 8) {  // the places of the partial sums: by image, warp, lane
+        __syncwarp();
+        const int total = warp_exclusive_scan(kw, n_img * nw);
+        for (int g = lane; g < n_slot; g += 32) slot_base[g] = kw[slot_first[g] * nw];
+        if (lane == 0) slot_base[n_slot] = total;
+      }
+      __syncthreads();
+      my = order[threadIdx.x];
+      units = my < n_item ? item_units[my] & 0xffff : 0;
+      w_units = __reduce_max_sync(0xffffffffu, units);
+      if (lane == 0) wunits[warp] = w_units;
+      __syncthreads();
+      batch0 = batches = quarter0 = 0;
+      for (int w = 0; w < nw; w++) {
+        const int u = wunits[w];
+        if (w < warp) {
+          batch0 += u;
+          if ((w & 3) == (warp & 3)) quarter0 += u;
+        }
+        batches += u;
+      }
+      n_part = slot_base[n_slot];
+      if (step == 1 || batches <= min(p.list_batches, n_part / 16 + 2 * nw)) break;
+      order[threadIdx.x] = n_item;
+      __syncthreads();
     }
-    const int key0 = kSortKeys - 32 - (((cnt[5] >> shift) >> 5) << 5);
-    __syncthreads();
-    if (warp == 0) {
-      warp_exclusive_scan(hist + key0 * nw, (kSortKeys - key0) * nw);
-    } else if (warp == 1) {  // the places of the partial sums: by image, warp, lane
-      const int total = warp_exclusive_scan(kw, n_img * nw);
-      for (int g = lane; g < n_slot; g += 32) slot_base[g] = kw[slot_first[g] * nw];
-      if (lane == 0) slot_base[n_slot] = total;
-    }
-    __syncthreads();
-    order[hist[key * nw + warp] + __popc(same & ((1u << lane) - 1u))] = threadIdx.x;
+    const ListItem item(my < n_item ? my : 0, ncol, nlc, nq, nzo);
     {  // place of every run's first partial sum
       int i = 0;
-      int2 r = units ? runs[0] : make_int2(1023, 0);
+      int2 r = own_units ? runs[0] : make_int2(1023, 0);
       for (int base = 0; base < n_img; base += 32) {
         const int k = base + lane;
         const int next = k + 1 < n_img || warp + 1 < nw ? (k < n_img ? kw[k * nw + warp + 1] : 0) : slot_base[n_slot];
@@ -821,24 +876,6 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
       }
     }
     __syncthreads();
-    const int my = order[threadIdx.x];
-    const bool has_item = my < n_item;
-    const ListItem item(has_item ? my : 0, ncol, nlc, nq, nzo);
-    units = has_item ? item_units[my] & 0xffff : 0;
-    const int w_units = __reduce_max_sync(0xffffffffu, units);
-    if (lane == 0) wunits[warp] = w_units;
-    __syncthreads();
-    // batches (units of a warp's 32 lanes) before this warp's, and units before it in its quarter
-    int batch0 = 0, batches = 0, quarter0 = 0;
-    for (int w = 0; w < nw; w++) {
-      const int u = wunits[w];
-      if (w < warp) {
-        batch0 += u;
-        if ((w & 3) == (warp & 3)) quarter0 += u;
-      }
-      batches += u;
-    }
-    const int n_part = slot_base[n_slot];
     bool overflow = cnt[2] || batches > p.list_batches || n_part > p.part_total;
     if constexpr (PAIR) {  // both CTAs take the capacity branch together
       if (threadIdx.x == 0) {
@@ -1096,9 +1133,9 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
 #pragma unroll
         for (int d = 1; d <= O; d++) cys[d] = splat(ISO ? p.czf[d] : p.cyf[d]);
         // the quad at row ybB + i of P and U, and P's row 7 further on; all lanes make ylen steps
-        unsigned aP = sP + 16u * (unsigned)(zB * PS4 + ql + pofs4 + ybB * nq);
+        unsigned aP = sP + 16u * (unsigned)(zB * PS4 + qB + pofs4 + ybB * nq);
         unsigned aN = aP + (unsigned)((O + 1) * RB);
-        unsigned aU = sU + 16u * (unsigned)(zB * PS4 + ql + uofs4 + ybB * nq);
+        unsigned aU = sU + 16u * (unsigned)(zB * PS4 + qB + uofs4 + ybB * nq);
         const int live = yeB - ybB, above = ny - (O + 1) - ybB;
         // ring[j] holds row ybB - 6 + j; row y+7 and U of row y+1 load while row y computes
         float4 ring[W];

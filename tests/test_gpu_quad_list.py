@@ -1,7 +1,8 @@
 """The split-pass kernel's projector list at the sizes where it can go wrong: cubes of fewer planes
 than a unit has (3^3), of one plane range per column and of several, with and without pad points in
-the last quad, on one CTA and on a pair, and every channel set the Mg pseudopotential gives (s+p,
-s+d, p+d).
+the last quad, columns dealt to the lanes by bank class and (most nodes of the three smallest) by the
+number of units alone, on one CTA and on a pair, and every channel set the Mg pseudopotential gives
+(s+p, s+d, p+d).
 
 Tolerance.  The first coefficients of the recurrence against the FP64 oracle: a_k and b_k are sums
 over stencil and projector terms of size up to 2 * 18 (h = 0.5), each rounded to FP32 (2^-24), about
