@@ -92,8 +92,8 @@ long long quad_table_float4(const TypeDesc &td) {
 }
 
 namespace {
-// One block row per (table, shift, channel): quads of the table's rows behind `shift` zeros, zeros
-// where the point lies outside the support sphere.
+// One block row per table: for every shift, quads of the table's rows behind `shift` zeros, zeros where
+// the point lies outside the support sphere; the planes and channels of a quad next to one another.
 __global__ void quad_tables_kernel(const __grid_constant__ LanczosParams p, const QuadTable *__restrict__ tabs,
                                    const float *__restrict__ src, float4 *__restrict__ dst) {
   const QuadTable t = tabs[blockIdx.x];
@@ -101,8 +101,8 @@ __global__ void quad_tables_kernel(const __grid_constant__ LanczosParams p, cons
   const int row = lq::quad_table_row(td), chan = lq::quad_table_channel(td);
   const int nch = __popc(td.chan_mask), fvol = td.fx * td.fy * td.fz;
   for (int e = threadIdx.x + blockDim.x * blockIdx.y; e < 4 * nch * chan; e += blockDim.x * gridDim.y) {
-    const int shift = e / (nch * chan), r = e - shift * nch * chan, c = r / chan, i = r - c * chan;
-    const int q = i % row, ly = i / row % td.fy, lz = i / (row * td.fy);
+    const int shift = e / (nch * chan), r = e - shift * nch * chan, c = r % nch, lz = r / nch % td.fz;
+    const int i = r / (nch * td.fz), q = i % row, ly = i / row;
     const float dy = fmaf(p.hyf, float(ly), t.oy), dz = fmaf(p.hzf, float(lz), t.oz);
     float v[4];
     for (int j = 0; j < 4; j++) {

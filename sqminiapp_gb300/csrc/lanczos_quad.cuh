@@ -214,8 +214,8 @@ __device__ __forceinline__ DF df_all_reduce(const float2 *red, int nw) {
 // writes its 8 quads at once if they are of 8 classes: the list's columns and pass B's are dealt to the
 // lanes that way (bank_slot).  Dealt by their number of units alone, over planes whose banks follow
 // on one another, a gather and a scatter of 27^3 took 7800 shared-memory wavefronts instead of 3450, of
-// 29^3 12000 instead of 4700: 39304 nodes of 27^3 and 40 steps 191.8 -> 179.7 ms, 17800 of 29^3 114.4 ->
-// 107.4 ms, 4864 of 33^3 on pairs 115.5 -> 110.7 ms (whole calls).
+// 29^3 12000 instead of 4700: 39304 nodes of 27^3 and 40 steps 191.8 -> 179.7 ms, 12001 of 29^3 and 50
+// steps 114.4 -> 107.4 ms, 9001 of 33^3 on pairs 115.5 -> 110.7 ms (whole calls).
 __host__ __device__ constexpr int quad_plane_floats(int ny, int pitch) {
   return (ny * pitch + 31) / 32 * 32;
 }
@@ -279,7 +279,9 @@ __host__ __device__ constexpr int list_scratch_bytes(int max_img, int nw) {
 }
 // The radial tables of this kernel hold whole quads: rows of the box's points behind `shift` zeros
 // (four copies, shift 0..3: the image's box start modulo 4 picks the one whose quads are the cube's),
-// zeros outside the support.  Quads of a row, and of a channel.
+// zeros outside the support.  The planes and channels of a column of quads lie next to one another
+// ([row][quad][plane][channel]): a unit is one run of memory, half the sectors of a plane by plane
+// layout.  Quads of a row, and of a channel.
 __host__ __device__ inline int quad_table_row(const TypeDesc &td) { return (td.fx + 6) / 4; }
 __host__ __device__ inline int quad_table_channel(const TypeDesc &td) {
   return quad_table_row(td) * td.fy * td.fz;
@@ -459,16 +461,16 @@ struct ListRun {
   int a, b;
   __device__ __forceinline__ int units() const { return (max(b - a, 0) + kRun - 1) / kRun; }
 };
-// Item t of the list: chunk t / columns of column t % columns.
+// Item t of the list: chunk t % chunks of column t / chunks, so that a warp's items lie in few rows.
 struct ListItem {
   int index, column;  // t, and the quad index in a plane
   int zb, ze;   // its planes, from the first owned one
   int top;      // units end here: ze, or kRun in a cube of fewer planes (that many are allocated)
   float x, y;   // cube coordinates of the column's first point
-  __device__ __forceinline__ ListItem(int t, int columns, int chunks, int nq, int planes) {
-    const int chunk = t / columns;
+  __device__ __forceinline__ ListItem(int t, int chunks, int nq, int planes) {
+    column = t / chunks;
+    const int chunk = t - column * chunks;
     index = t;
-    column = t - chunk * columns;
     const int row = column / nq;
     x = float(4 * (column - row * nq));
     y = float(row);
@@ -476,26 +478,24 @@ struct ListItem {
     ze = planes * (chunk + 1) / chunks;
     top = max(ze, zb + kRun);
   }
-  __device__ __forceinline__ ListRun run(const LanczosParams &p, const ImgRow *row, int nx, float ih) const {
+  // A run may be longer than the support (T is zero there), but no quad lies outside the image's box.
+  __device__ __forceinline__ ListRun run(const LanczosParams &p, const ImgRow *row, float ih) const {
     const ImgRow g = load_row(row);
     const TypeDesc &td = p.types[g.type()];
     const float fx = x - g.bx, fy = y - g.by;
-    float near = 3e38f;  // smallest dx^2 of the points in the cube and the box
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const float f = fx + float(i), dx = fmaf(p.hxf, f, g.ox);
-      if (f >= 0.f && f < float(td.fx) && x + float(i) < float(nx)) near = fminf(near, dx * dx);
-    }
-    const float dy = fmaf(p.hyf, fy, g.oy), rest = td.support_r2_f32 - near - dy * dy;
-    if (!(rest >= 0.f) || fy < 0.f || fy >= float(td.fy)) return ListRun{0, 0};
-    // |oz + hz (z - bz)| <= sqrt(rest), a touch wider: T is masked point by point
-    const float half = sqrtf(rest);
+    const float d0 = fmaf(p.hxf, fx, g.ox), d1 = d0 + p.hxf, d2 = d1 + p.hxf, d3 = d2 + p.hxf;
+    const float near = fminf(fminf(fabsf(d0), fabsf(d1)), fminf(fabsf(d2), fabsf(d3)));
+    const float dy = fmaf(p.hyf, fy, g.oy), rest = td.support_r2_f32 * (1.f + 1e-5f) - near * near - dy * dy;
+    const bool meets = rest >= 0.f && fx > -4.f && fx < float(td.fx) && fy >= 0.f && fy < float(td.fy);
+    // |oz + hz (z - bz)| <= sqrt(rest), a touch wider
+    float half;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(half) : "f"(fmaxf(rest, 0.f)));
     const float low = fmaf(-half - g.oz, ih, -1e-3f), high = fmaf(half - g.oz, ih, 1e-3f);
     const int bz = (int)g.bz;
     ListRun r;
     r.a = max(zb, bz + max(0, (int)ceilf(low)));
     r.b = min(ze, bz + min(td.fz, (int)floorf(high) + 1));
-    return r.b > r.a ? r : ListRun{0, 0};
+    return meets && r.b > r.a ? r : ListRun{0, 0};
   }
 };
 // Exclusive scan of n integers in place by one warp; returns their sum.
@@ -766,14 +766,17 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
     const int n_slot = cnt[1];
 
     // ---- runs of every item (thread t: item t), kept in the scratch slice; units per (image, warp)
-    // and per item.  The warp's lanes share the images whose boxes meet the bounds of its columns ----
+    // and per item.  The warp's lanes share the images whose boxes meet the bounds of its columns; both
+    // plane ranges of a column in one warp make those bounds few rows (a warp that held the end of one
+    // range and the start of the next took all 63 images, and the CTA waited for it).  The whole build of
+    // a node of 27^3 and 63 images: 111K -> 58K cycles, 40 steps 1.36M ----
     int *order = scratch, *kw = order + 32 * nw;
     int *item_units = kw + maxi * nw;
     int2 *runs = reinterpret_cast<int2 *>(grun) + threadIdx.x;  // run i: + i * blockDim.x
     int units = 0;
-    {
+    {  // and its first unit's place among the warp's of the image
       const bool mine = threadIdx.x < n_item;
-      const ListItem it(mine ? threadIdx.x : 0, ncol, nlc, nq, nzo);
+      const ListItem it(mine ? threadIdx.x : 0, nlc, nq, nzo);
       const int row = it.column / nq;
       const int r0 = __reduce_min_sync(0xffffffffu, mine ? row : ny), r1 = __reduce_max_sync(0xffffffffu, mine ? row : -1);
       const int z0 = __reduce_min_sync(0xffffffffu, mine ? it.zb : nzo), z1 = __reduce_max_sync(0xffffffffu, mine ? it.ze : 0);
@@ -787,15 +790,30 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
           near = (int)g.by <= r1 && (int)g.by + td.fy > r0 && (int)g.bz < z1 && (int)g.bz + td.fz > z0;
         }
         int total = 0;  // of image k
-        for (unsigned todo = __ballot_sync(0xffffffffu, near); todo; todo &= todo - 1) {
-          const int src = __ffs(todo) - 1;
-          const ListRun r = mine ? it.run(p, rows + base + src, nx, ihz) : ListRun{0, 0};
-          const int n = r.units(), t = __reduce_add_sync(0xffffffffu, n);
-          if (lane == src) total = t;
-          if (n) {
-            runs[(size_t)blockDim.x * n_run++] = make_int2((base + src) | (r.a << 10) | (r.b << 17), 0);
-            units += n;
+        auto keep = [&](int k, ListRun r, int place) {
+          if (!r.units()) return;
+          runs[(size_t)blockDim.x * n_run++] = make_int2(k | (r.a << 10) | (r.b << 17), place);
+          units += r.units();
+        };
+        for (unsigned todo = __ballot_sync(0xffffffffu, near); todo;) {  // two images at once
+          const int s0 = __ffs(todo) - 1;
+          todo &= todo - 1;
+          const int s1 = todo ? __ffs(todo) - 1 : 32;
+          todo &= todo - 1;
+          const ListRun q0 = it.run(p, rows + base + s0, ihz), q1 = it.run(p, rows + base + (s1 & 31), ihz);
+          const ListRun r0 = mine ? q0 : ListRun{0, 0}, r1 = mine && s1 < 32 ? q1 : ListRun{0, 0};
+          const int n = r0.units() | r1.units() << 16;
+          int incl = n;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
           }
+          const int all = __shfl_sync(0xffffffffu, incl, 31);
+          total = lane == s0 ? all & 0xffff : lane == s1 ? all >> 16 : total;
+          incl -= n;
+          keep(base + s0, r0, incl & 0xffff);
+          keep(base + s1, r1, incl >> 16);
         }
         if (k < n_img) kw[k * nw + warp] = total;
       }
@@ -811,11 +829,11 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
     int my, w_units, n_part, batch0, batches, quarter0;  // batches before this warp's, units before it in its quarter
     for (int step = 8;; step = 1) {
       if ((int)threadIdx.x < n_item) {
-        const int r = step == 1 ? 0 : (int)threadIdx.x % ncol & 7;
+        const int r = step == 1 ? 0 : (int)threadIdx.x / nlc & 7;
         int rank = 0;
-        for (int c = 0; c < n_item; c += ncol)
+        for (int c = r * nlc; c < (r + 1) * nlc; c++)
 #pragma unroll 4
-          for (int t = c + r; t < c + ncol; t += step) {
+          for (int t = c; t < n_item; t += step * nlc) {
             const int n = item_units[t] & 0xffff;
             rank += n > own_units || (n == own_units && t < (int)threadIdx.x);
           }
@@ -849,33 +867,7 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
       order[threadIdx.x] = n_item;
       __syncthreads();
     }
-    const ListItem item(my < n_item ? my : 0, ncol, nlc, nq, nzo);
-    {  // place of every run's first partial sum
-      int i = 0;
-      int2 r = own_units ? runs[0] : make_int2(1023, 0);
-      for (int base = 0; base < n_img; base += 32) {
-        const int k = base + lane;
-        const int next = k + 1 < n_img || warp + 1 < nw ? (k < n_img ? kw[k * nw + warp + 1] : 0) : slot_base[n_slot];
-        unsigned todo = __ballot_sync(0xffffffffu, k < n_img && next != kw[k * nw + warp]);
-        for (; todo; todo &= todo - 1) {
-          const int q = base + __ffs(todo) - 1;
-          const bool on = (r.x & 1023) == q;
-          const int n = on ? ListRun{(r.x >> 10) & 127, r.x >> 17}.units() : 0;
-          int incl = n;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += t;
-          }
-          if (on) {
-            runs[(size_t)blockDim.x * i].y = kw[q * nw + warp] + incl - n;
-            i++;
-            r = i < (item_units[threadIdx.x] >> 16) ? runs[(size_t)blockDim.x * i] : make_int2(1023, 0);
-          }
-        }
-      }
-    }
-    __syncthreads();
+    const ListItem item(my < n_item ? my : 0, nlc, nq, nzo);
     bool overflow = cnt[2] || batches > p.list_batches || n_part > p.part_total;
     if constexpr (PAIR) {  // both CTAs take the capacity branch together
       if (threadIdx.x == 0) {
@@ -887,7 +879,8 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
     } else {
       // the next node, read by every thread after this node's last barrier (the previous
       // value was read before the barriers above)
-      if (threadIdx.x == 0) cnt[3] = atomicAdd(status + 1, 1);
+      // (by the last warp, which has the fewest units)
+      if (threadIdx.x == blockDim.x - 1) cnt[3] = atomicAdd(status + 1, 1);
     }
     if (overflow) {  // capacity exceeded: report, NaN coefficients
       if (threadIdx.x == 0) atomicOr(status, kStatusCapacity);
@@ -910,57 +903,57 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
       const int2 *mine = reinterpret_cast<const int2 *>(grun) + item.index;
       const bool k1 = (int)item.x + 1 < nx, k2 = (int)item.x + 2 < nx, k3 = (int)item.x + 3 < nx;
       const int xq = (int)item.x >> 2;
-      int left = 0, a = 0, b = 0, place = 0, cmask = 0, plane = 0;
+      const int n_run = my < n_item ? item_units[my] >> 16 : 0;
+      int left = 0, a = 0, b = 0, place = 0, cmask = 0, nc = 0;
       const float4 *tq = qtables;  // the column's quad of plane 0 of the box, channel 0
-      long long chan = 0;
       ImgRow g{};
       int i = 0;
-      for (int u = 0; u < w_units; u++) {
-        float4 T[NCH][kRun];
-        float4 meta = make_float4(__uint_as_float(unit_word(0, item.zb, 0)), 0.f, 0.f, 0.f);
+      auto unit = [&](int u, float4 (&T)[NCH][kRun], float4 &meta) {
+        meta = make_float4(__uint_as_float(unit_word(0, item.zb, 0)), 0.f, 0.f, 0.f);
+        const bool on = u < units;
+        if (on && left == 0) {
+          const int2 r = mine[(size_t)blockDim.x * i++];
+          const ListRun run{(r.x >> 10) & 127, r.x >> 17};
+          a = run.a;
+          b = run.b;
+          left = run.units();
+          place = r.y + kw[(r.x & 1023) * nw + (item.index >> 5)];
+          g = load_row(rows + (r.x & 1023));
+          const TypeDesc &td = p.types[g.type()];
+          cmask = td.chan_mask;
+          nc = __popc(cmask);
+          tq = qtables +
+               (g.tab + (((int)item.y - (int)g.by) * quad_table_row(td) + xq - ((int)g.bx >> 2)) * td.fz * nc);
+        }
+        const int z0 = on ? min(a, item.top - kRun) : item.zb;
+        if (on)
+          meta = make_float4(__uint_as_float(unit_word(g.slot(), z0, place)), fmaf(p.hxf, item.x - g.bx, g.ox),
+                             fmaf(p.hyf, item.y - g.by, g.oy), fmaf(p.hzf, float(z0) - g.bz, g.oz));
+        const float4 *tz = tq + (z0 - (int)g.bz) * nc;
+        int c = 0, ch = 0;
+#pragma unroll
+        for (int l = 0; l < 4; l++) {
+          if (!(MASK & (1 << l))) continue;
+          const bool have = on && (cmask & (1 << l));
+#pragma unroll
+          for (int q = 0; q < kRun; q++)  // planes [a, b) of the unit's
+            T[c][q] = ldg_quad_if(have && z0 + q >= a && z0 + q < b, tz + q * nc + ch);
+          ch += have ? 1 : 0;
+          c++;
+        }
+        a = on ? z0 + kRun : a;
+        place += on;
+        left -= on;
+      };
+      auto store = [&](int u, float4 (&T)[NCH][kRun], float4 meta) {
 #pragma unroll
         for (int c = 0; c < NCH; c++)
 #pragma unroll
-          for (int q = 0; q < kRun; q++) T[c][q] = zero4;
-        if (u < units) {
-          if (left == 0) {  // the item's next image
-            const int2 r = mine[(size_t)blockDim.x * i++];
-            const ListRun run{(r.x >> 10) & 127, r.x >> 17};
-            a = run.a;
-            b = run.b;
-            left = run.units();
-            place = r.y;
-            g = load_row(rows + (r.x & 1023));
-            const TypeDesc &td = p.types[g.type()];
-            cmask = td.chan_mask;
-            plane = quad_table_row(td) * td.fy;
-            chan = quad_table_channel(td);
-            tq = qtables + (g.tab + ((int)item.y - (int)g.by) * quad_table_row(td) + xq - ((int)g.bx >> 2));
+          for (int q = 0; q < kRun; q++) {  // pad points
+            T[c][q].y = k1 ? T[c][q].y : 0.f;
+            T[c][q].z = k2 ? T[c][q].z : 0.f;
+            T[c][q].w = k3 ? T[c][q].w : 0.f;
           }
-          const int z0 = min(a, item.top - kRun);
-          meta = make_float4(__uint_as_float(unit_word(g.slot(), z0, place)), fmaf(p.hxf, item.x - g.bx, g.ox),
-                             fmaf(p.hyf, item.y - g.by, g.oy), fmaf(p.hzf, float(z0) - g.bz, g.oz));
-          const float4 *tz = tq + (z0 - (int)g.bz) * plane;
-          int c = 0, ch = 0;
-#pragma unroll
-          for (int l = 0; l < 4; l++) {
-            if (!(MASK & (1 << l))) continue;
-            const bool have = cmask & (1 << l);
-#pragma unroll
-            for (int q = 0; q < kRun; q++) {  // planes [a, b) of the unit's
-              float4 t = ldg_quad_if(have && z0 + q >= a && z0 + q < b, tz + ch * chan + q * plane);
-              t.y = k1 ? t.y : 0.f;
-              t.z = k2 ? t.z : 0.f;
-              t.w = k3 ? t.w : 0.f;
-              T[c][q] = t;
-            }
-            ch += have ? 1 : 0;
-            c++;
-          }
-          a = z0 + kRun;
-          place++;
-          left--;
-        }
         __syncwarp();
         if (u < tm_units) {
 #pragma unroll
@@ -973,6 +966,15 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
             for (int q = 0; q < kRun; q++) wT[((u * NCH + c) * kRun + q) * 32] = T[c][q];
           wmeta[32 * u] = meta;
         }
+      };
+      constexpr int kAtOnce = MAXT <= 384 && NCH <= 2 ? 2 : 1;  // units whose table loads are in flight together
+      for (int u = 0; u < w_units; u += kAtOnce) {
+        float4 T[kAtOnce][NCH][kRun], meta[kAtOnce];
+#pragma unroll
+        for (int k = 0; k < kAtOnce; k++) unit(u + k, T[k], meta[k]);
+#pragma unroll
+        for (int k = 0; k < kAtOnce; k++)
+          if (u + k < w_units) store(u + k, T[k], meta[k]);
       }
       tmem_wait_st();
     }
