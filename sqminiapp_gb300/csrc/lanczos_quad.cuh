@@ -57,7 +57,7 @@
 // most of the FP32 error (weights 6e-6 -> 4e-7 and the lowest Ritz value 5e-7 -> 5e-8 Ha on a 27^3
 // cube without projectors, the diagonal's share of the weights' rounding included).
 //
-// Memory traffic.  Pass A reads Veff from L2 two planes ahead.  Nodes after the first round come
+// Memory traffic.  Pass A reads Veff from L2 one plane ahead.  Nodes after the first round come
 // from a device-side queue.
 //
 // CTA pair (PAIR, lanczos_quad_pair_kernel): one node per cluster of two CTAs for cubes whose
@@ -661,7 +661,7 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
       const int c = grp / nzo, r = (c * ylen * nq + ql) & 7;
       int rank = (ql >> 3) * nzo + grp % nzo;
       for (int i = 0; i < c; i++) rank += of_class(i, r) * nzo;
-      scratch[bank_slot(r, rank, (int)blockDim.x >> 3, [&](int i) {
+      scratch[bank_slot(r, rank, (nchB * nzo * nq + 31) / 32 * 4, [&](int i) {  // as few warps as hold them
         int n = 0;
         for (int k = 0; k < nchB; k++) n += of_class(k, i) * nzo;
         return n;
@@ -1061,14 +1061,10 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
         // x neighbours: the upper half of quad q-2, quads q-1 and q+1, the lower half of q+2
         float2 xm2 = make_float2(0.f, 0.f), xp2 = make_float2(0.f, 0.f);
         float4 xm1 = zero4, xp1 = zero4;
-        // U one plane ahead, Veff (from L2) two; the 16-warp budget has no registers for either
-        constexpr bool kAhead = MAXT <= 384;
-        float4 nuo = zero4, dv1 = zero4, dv2 = zero4;
-        if constexpr (kAhead) {
-          nuo = lds_quad(aU);
-          dv1 = __ldg(vrow);
-          dv2 = __ldg(vrow + min(1, live - 1) * VPS4);
-        }
+        // Veff (from L2) one plane ahead; P and U of a plane as it begins, which the arithmetic of the
+        // other warps covers.  With Veff two planes and U one ahead (13 registers more and copies between
+        // them) 4864 nodes took 20.5 instead of 20.1 ms at 27^3, 57.0 instead of 54.9 on pairs at 33^3
+        float4 dv1 = __ldg(vrow);
         for (int i0 = 0; i0 < zlen; i0 += W) {
 #pragma unroll
           for (int s = 0; s < W; s++) {
@@ -1081,17 +1077,8 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
             lds_quad_if<16>(hp1, aP, xp1);
             lds_pair_if<32>(hp2, aP, xp2);
             const float4 c = RING(0);
-            float4 dv, uo;
-            if constexpr (kAhead) {
-              dv = dv1;
-              dv1 = dv2;
-              dv2 = __ldg(vrow + min(i + 2, live - 1) * VPS4);
-              uo = nuo;
-              lds_quad_if<0>(i + 1 < live, aU + (unsigned)PB, nuo);
-            } else {
-              dv = __ldg(vrow + min(i, live - 1) * VPS4);
-              uo = lds_quad(i < live ? aU : sZ);
-            }
+            const float4 dv = dv1, uo = lds_quad(i < live ? aU : sZ);
+            dv1 = __ldg(vrow + min(i + 1, live - 1) * VPS4);
             float2 h01 = mul2(lo(dv), lo(c)), h23 = mul2(hi(dv), hi(c));
 #pragma unroll
             for (int d = 1; d <= O; d++) {
@@ -1134,27 +1121,25 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
         float2 cys[O + 1];
 #pragma unroll
         for (int d = 1; d <= O; d++) cys[d] = splat(ISO ? p.czf[d] : p.cyf[d]);
-        // the quad at row ybB + i of P and U, and P's row 7 further on; all lanes make ylen steps
+        // the quad at row ybB + i of P and U, and P's row 6 further on; all lanes make ylen steps
         unsigned aP = sP + 16u * (unsigned)(zB * PS4 + qB + pofs4 + ybB * nq);
-        unsigned aN = aP + (unsigned)((O + 1) * RB);
+        unsigned aN = aP + (unsigned)(O * RB);
         unsigned aU = sU + 16u * (unsigned)(zB * PS4 + qB + uofs4 + ybB * nq);
-        const int live = yeB - ybB, above = ny - (O + 1) - ybB;
-        // ring[j] holds row ybB - 6 + j; row y+7 and U of row y+1 load while row y computes
+        const int live = yeB - ybB, above = ny - O - ybB;
+        // before the step of row y, ring[j] holds row y - 6 + j (mod W); y + 6 joins at its start
         float4 ring[W];
 #pragma unroll
-        for (int j = 0; j < W; j++) {
+        for (int j = 0; j < W - 1; j++) {
           const int yq = ybB - O + j;
           ring[j] = lds_quad(yq >= 0 && yq < ny ? aP + (unsigned)((j - O) * RB) : sZ);
         }
-        float4 nuo = lds_quad(aU);
         for (int i0 = 0; i0 < ylen; i0 += W) {
 #pragma unroll
           for (int s = 0; s < W; s++) {
             const int i = i0 + s;
             if (i >= ylen) break;
-            const float4 uo = nuo;
-            const float4 nring = lds_quad(i < above ? aN : sZ);
-            lds_quad_if<0>(i + 1 < live, aU + (unsigned)RB, nuo);
+            ring[(s + W - 1) % W] = lds_quad(i < above ? aN : sZ);
+            const float4 uo = lds_quad(i < live ? aU : sZ);
 #define RING(dd) ring[(s + (dd) + O) % W]
             float2 h01 = mul2(cys[1], add2(lo(RING(-1)), lo(RING(1))));
             float2 h23 = mul2(cys[1], add2(hi(RING(-1)), hi(RING(1))));
@@ -1169,7 +1154,6 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
             sts_quad_if(i < live, aU, make_float4(n01.x, n01.y, n23.x, n23.y));
             const float2 pa = fma2(lo(c), h01, mul2(hi(c), h23));
             ka.add(i < live ? pa.x + pa.y : 0.f);
-            ring[s] = nring;  // row y-6 leaves, row y+7 joins
             aN += (unsigned)RB;
             aU += (unsigned)RB;
           }
