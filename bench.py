@@ -70,7 +70,7 @@ def parse_args():
     p.add_argument("--kernel", type=int, choices=[0, 1, 2], default=0,
                    help="FP32 Lanczos kernel: 0 automatic, 1 single-pass, 2 split-pass")
     p.add_argument("--tile", type=int, default=0,
-                   help="split-pass kernel tile (z-/y-ranges per row); 0 autotuned")
+                   help="split-pass kernel tile (z-/y-ranges per row); 0 automatic")
     p.add_argument("--list-format", type=int, choices=[0, 1, 2], default=0,
                    help="projector-list records of the main workload: 0 automatic, 1 full, "
                         "2 compact")

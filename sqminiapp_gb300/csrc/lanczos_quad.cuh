@@ -6,11 +6,11 @@
 // src/lsdft_matvec.cc:25-149); FP32 vectors, corrected operator, full projector records.
 //
 // Layout.  P and U are both [nz][ny][pitch] floats in shared memory, pitch = 4*ceil(nx/4),
-// planes padded to a bank-friendly stride (quad_plane_floats): every row starts on a 16-byte
-// boundary and holds whole float4 quads; the pad columns [nx, pitch) and plane pads stay zero.  There are no zero rows or columns between rows: neighbours outside
-// the cube are never loaded (x: the quad loads are predicated off at the row ends; y and z:
-// the register rings start and end with zeros).  A point's P and U indices are the same,
-// z*PS + y*pitch + x.
+// planes a multiple of all banks apart (quad_plane_floats): every row starts on a 16-byte boundary
+// and holds whole float4 quads; the pad columns [nx, pitch) and plane pads stay zero.  There are no
+// zero rows or columns between rows: neighbours outside the cube are never loaded (x: the quad loads
+// are predicated off at the row ends; y and z: a quad of zeros stands for them).  A point's P and U
+// indices are the same, z*PS + y*pitch + x.
 //
 // Stencil, split by axis so that two of the three axes come from registers:
 //   pass A  a thread owns one quad (x..x+3) of row y over a z-range and walks z with a
@@ -20,15 +20,15 @@
 //           forms U <- s (diag + Dz + Dx) P - gamma U;
 //   pass B  a thread owns one quad of plane z over a y-range and walks y with a 13-row
 //           register ring: U += s Dy P.
-// Eight consecutive threads own the quads of one row (pass A) or one plane (pass B), so a
-// quarter-warp's float4 accesses cover one contiguous row: no bank conflicts.
+// Consecutive threads own consecutive quads in pass A; pass B's columns are dealt to the lanes by the
+// bank they begin in: hardly any bank conflicts in either.
 //
 // Projector list.  Its unit is (image, column of quads, four planes): T_l of four quads above one
 // another (zero outside the support), and one word with the image, the first plane and the place of
 // the unit's partial sums; chi_lm = T_l P_lm(x,y,z) is formed while streaming, over a column with the
 // same x and y for every plane.  A thread owns one column over a range of planes and all its units
-// (dealt out by their number, so that the lanes of a warp have equally many): no two threads meet on a
-// quad, the scatter needs no atomics, and every run gives the same result.  The list is built once per
+// (dealt out by bank and number, so that the lanes of a warp have equally many and read eight banks at
+// once): no two threads meet on a quad, the scatter needs no atomics, and every run gives the same result.  The list is built once per
 // node and lives in the SM's tensor memory, which this kernel does not need for anything else
 // (tcgen05.ld: no L2 round trip, no shared memory); what exceeds its 512 columns goes to a slice of
 // global scratch.  The gather writes four (s+p) partial sums per unit, ordered by atom, to shared
