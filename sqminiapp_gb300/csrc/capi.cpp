@@ -366,9 +366,10 @@ void plan_engine(sq_handle *h, int smem_optin, int l2_bytes) {
     };
     // Tile (plane / row ranges per thread walk) and CTAs per SM: the most threads in the stencil
     // passes, a walk of L planes counted as L / (L + 5) for the 12 it loads first and the 16-warp
-    // kernels, with 128 registers, as 0.85.  Measured with every tile (ms per 3648 nodes, 20 steps; the
-    // chosen one first): 13^3 2.20 (tile 2, 3 CTAs), 2.40, 2.74; 17^3 3.50 (2, 2 CTAs), 4.10, 4.20; 19^3
-    // 3.97 (2, 2 CTAs), 4.61; 21^3 5.42 (3), 5.78, 6.06; 23^3 6.39 (3), 7.15; 27^3 9.74 (2), 13.20.
+    // kernels, with 128 registers, as 0.78.  Measured with every tile (ms per 3648 nodes, 20 steps; the
+    // chosen one first): 9^3 0.81 (tile 3), 0.88, 0.98, 1.03; 13^3 1.67 (2, 3 CTAs), 1.72, 1.95; 17^3 2.76
+    // (2, 2 CTAs), 3.16, 3.24; 19^3 3.17 (2, 2 CTAs), 3.69; 21^3 4.25 (3), 4.55, 5.11; 23^3 5.69 (3, 16
+    // warps), 5.87; 27^3 7.88 (2), 11.11.
     double best = 0.0;
     sq::LanczosParams chosen = q;
     for (int tile = h->opt.tile > 0 ? h->opt.tile : 1; !wide && tile <= std::max(4, h->opt.tile); tile++) {
@@ -383,7 +384,7 @@ void plan_engine(sq_handle *h, int smem_optin, int l2_bytes) {
         const int ctas = sq::lanczos_quad_place_partials(t, block, smem_optin);
         const double walk = (double)((p.nz + tile - 1) / tile);
         const double score = (double)ctas * (p.ny * (t.pitch / 4) * tile) * walk / (walk + 5.0) *
-                             (block > 384 ? 0.85 : 1.0);
+                             (block > 384 ? 0.78 : 1.0);
         if (score > best) {
           best = score;
           chosen = t;
