@@ -558,6 +558,11 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
   constexpr int NCH = Chi::nch;
   constexpr int kTCols = 4 * kRun * NCH;  // tensor-memory columns of a unit's T
   constexpr int kPart = (NLM + 3) / 4;    // float4 of a unit's partial sums
+  // The arrays of P and U change places every step: the update writes one instead of two of them (the
+  // shared-memory data path is what the kernel waits for most).  4864 nodes of 29^3 and 50 steps 40.2 ->
+  // 38.6 ms; the 12-warp kernel, which has the registers to read the update's next quads ahead, gains
+  // nothing (27^3 20.05 and 20.15 ms); a CTA of a pair holds more planes of P than of U.
+  constexpr bool kSwap = !PAIR && MAXT > 384;
   const int nw = blockDim.x >> 5;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nx = p.nx, ny = p.ny, nz = p.nz, pitch = p.pitch;
@@ -993,7 +998,8 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
       }
     };
     // the item's column in P (owned planes) and U
-    const unsigned itemP = smem_addr(P4o) + 16u * (unsigned)item.column, itemU = sU + 16u * (unsigned)item.column;
+    const unsigned itemP = 16u * (unsigned)(item.column + (zo0 - pz0) * PS4), itemU = 16u * (unsigned)item.column;
+    unsigned aP0 = sP, aU0 = sU;  // the arrays of P and U (kSwap: they change places every step)
     __syncthreads();  // the scratch in U is read
     for (int e = threadIdx.x; e < (ncu >> 2); e += blockDim.x) U4[e] = zero4;
     {  // v_0: the unit vector at the cube centre, in every CTA that holds that plane of P
@@ -1022,7 +1028,7 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
         float4 T[NCH][kRun], meta;
         load_unit(u, T, meta);
         const unsigned w = __float_as_uint(meta.x);
-        unsigned a = itemP + (unsigned)((int)((w >> 10) & 63u) * PB);
+        unsigned a = aP0 + itemP + (unsigned)((int)((w >> 10) & 63u) * PB);
         float4 v[kRun];
 #pragma unroll
         for (int i = 0; i < kRun; i++, a += (unsigned)PB) v[i] = lds_quad(a);
@@ -1048,9 +1054,9 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
         const float4 *vrow = vq + (size_t)(K * p.EY + J + yA) * VRS4 + ql + (size_t)zbA * VPS4;
         // the quad at plane zbA + i of P and U, and P's plane 6 further on: all lanes make zlen
         // steps (a uniform loop), those past their range keep nothing
-        unsigned aP = sP + 16u * (unsigned)(row4 + zbA * PS4 + pofs4);
+        unsigned aP = aP0 + 16u * (unsigned)(row4 + zbA * PS4 + pofs4);
         unsigned aN = aP + (unsigned)(O * PB);
-        unsigned aU = sU + 16u * (unsigned)(row4 + zbA * PS4 + uofs4);
+        unsigned aU = aU0 + 16u * (unsigned)(row4 + zbA * PS4 + uofs4);
         const int live = zeA - zbA, above = nz - O - zbA;
         float4 ring[W];
 #pragma unroll
@@ -1122,9 +1128,9 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
 #pragma unroll
         for (int d = 1; d <= O; d++) cys[d] = splat(ISO ? p.czf[d] : p.cyf[d]);
         // the quad at row ybB + i of P and U, and P's row 6 further on; all lanes make ylen steps
-        unsigned aP = sP + 16u * (unsigned)(zB * PS4 + qB + pofs4 + ybB * nq);
+        unsigned aP = aP0 + 16u * (unsigned)(zB * PS4 + qB + pofs4 + ybB * nq);
         unsigned aN = aP + (unsigned)(O * RB);
-        unsigned aU = sU + 16u * (unsigned)(zB * PS4 + qB + uofs4 + ybB * nq);
+        unsigned aU = aU0 + 16u * (unsigned)(zB * PS4 + qB + uofs4 + ybB * nq);
         const int live = yeB - ybB, above = ny - O - ybB;
         // before the step of row y, ring[j] holds row y - 6 + j (mod W); y + 6 joins at its start
         float4 ring[W];
@@ -1251,7 +1257,7 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
           if (4 * i + 2 < NLM) q[4 * i + 2] = t.z;
           if (4 * i + 3 < NLM) q[4 * i + 3] = t.w;
         }
-        const unsigned a = itemU + (unsigned)((int)((w >> 10) & 63u) * PB);
+        const unsigned a = aU0 + itemU + (unsigned)((int)((w >> 10) & 63u) * PB);
         float4 v[kRun];
 #pragma unroll
         for (int i = 0; i < kRun; i++) v[i] = lds_quad(a + (unsigned)(i * PB));
@@ -1288,29 +1294,47 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
           dpeer = (zo0 - pq.pz0) * PS4;
           P4peer = cooperative_groups::this_cluster().map_shared_rank(P4, cr ^ 1);
         }
-        // the next quad's P and U are read before this quad's are written
-        float4 npv = zero4, nuv = zero4;
-        if (threadIdx.x < nown) {
-          npv = P4o[threadIdx.x];
-          nuv = U4[threadIdx.x];
-        }
-        for (int e = threadIdx.x; e < nown; e += blockDim.x) {
-          const float4 pv = npv, uv = nuv;
-          if (e + (int)blockDim.x < nown) {
-            npv = P4o[e + blockDim.x];
-            nuv = U4[e + blockDim.x];
+        if constexpr (kSwap) {
+          // w goes where U was, and P stays as the next U (scaled through gamma)
+          const float2 nahs2 = splat(-ak.hi * sc), nals2 = splat(-ak.lo * sc);
+          unsigned ap = aP0 + 16u * threadIdx.x, au = aU0 + 16u * threadIdx.x;
+          const unsigned step = 16u * blockDim.x;
+          for (int e = threadIdx.x; e < nown; e += blockDim.x) {
+            const unsigned at = au;
+            const float4 pv = lds_quad(ap), uv = lds_quad(au);
+            ap += step;
+            au += step;
+            const float2 w01 = fma2(nals2, lo(pv), fma2(nahs2, lo(pv), lo(uv)));
+            const float2 w23 = fma2(nals2, hi(pv), fma2(nahs2, hi(pv), hi(uv)));
+            sts_quad_if(true, at, make_float4(w01.x, w01.y, w23.x, w23.y));
+            const float2 q = fma2(w01, w01, mul2(w23, w23));
+            kb.add(q.x + q.y);
           }
-          const float2 v01 = mul2(lo(pv), sc2), v23 = mul2(hi(pv), sc2);
-          const float2 w01 = fma2(nal2, v01, fma2(nah2, v01, lo(uv)));
-          const float2 w23 = fma2(nal2, v23, fma2(nah2, v23, hi(uv)));
-          const float4 w4 = make_float4(w01.x, w01.y, w23.x, w23.y);
-          P4o[e] = w4;
-          if constexpr (PAIR) {
-            if (e >= h0 && e < h1) P4peer[e + dpeer] = w4;
+        } else {
+          // the next quad's P and U are read before this quad's are written
+          float4 npv = zero4, nuv = zero4;
+          if (threadIdx.x < nown) {
+            npv = P4o[threadIdx.x];
+            nuv = U4[threadIdx.x];
           }
-          U4[e] = make_float4(v01.x, v01.y, v23.x, v23.y);
-          const float2 q = fma2(w01, w01, mul2(w23, w23));
-          kb.add(q.x + q.y);
+          for (int e = threadIdx.x; e < nown; e += blockDim.x) {
+            const float4 pv = npv, uv = nuv;
+            if (e + (int)blockDim.x < nown) {
+              npv = P4o[e + blockDim.x];
+              nuv = U4[e + blockDim.x];
+            }
+            const float2 v01 = mul2(lo(pv), sc2), v23 = mul2(hi(pv), sc2);
+            const float2 w01 = fma2(nal2, v01, fma2(nah2, v01, lo(uv)));
+            const float2 w23 = fma2(nal2, v23, fma2(nah2, v23, hi(uv)));
+            const float4 w4 = make_float4(w01.x, w01.y, w23.x, w23.y);
+            P4o[e] = w4;
+            if constexpr (PAIR) {
+              if (e >= h0 && e < h1) P4peer[e + dpeer] = w4;
+            }
+            U4[e] = make_float4(v01.x, v01.y, v23.x, v23.y);
+            const float2 q = fma2(w01, w01, mul2(w23, w23));
+            kb.add(q.x + q.y);
+          }
         }
         const DF bp = df_warp_sum(df_of(kb));
         if (lane == 0) red_b[warp] = make_float2(bp.hi, bp.lo);
@@ -1337,10 +1361,15 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
       // gamma = <s' w, H s P> / |s P|^2 = s' |w|^2 / (s^2 |P|^2)
       const float nsc = unit_scale(b2.hi);
       const DF g = df_div(b2, n2);
-      const float gs = nsc / (sc * sc);
+      const float gs = kSwap ? nsc / sc : nsc / (sc * sc);  // kSwap: U is P = v / s
       gam = DF{g.hi * gs, g.lo * gs};
       n2 = b2;
       sc = nsc;
+      if constexpr (kSwap) {
+        const unsigned t = aP0;
+        aP0 = aU0;
+        aU0 = t;
+      }
     }
     __syncthreads();
     if (cr == 0)
