@@ -301,6 +301,7 @@ void plan_engine(sq_handle *h, int smem_optin, int l2_bytes) {
   p.hzf = (float)p.hz;
   p.cdiag = s.c[0][0] + s.c[1][0] + s.c[2][0];
   p.cdiagf = (float)p.cdiag;
+  p.hshift = p.cdiag;
   for (int q = 0; q <= sq::kStencilHalf; q++) {
     p.cx[q] = s.c[0][q];
     p.cy[q] = s.c[1][q];
@@ -308,6 +309,10 @@ void plan_engine(sq_handle *h, int smem_optin, int l2_bytes) {
     p.cxf[q] = (float)p.cx[q];
     p.cyf[q] = (float)p.cy[q];
     p.czf[q] = (float)p.cz[q];
+    // hshift also takes up what the FP32 stencil weights lose on a constant vector, so that their
+    // rounding does not shift the low end of the spectrum
+    if (q > 0)
+      p.hshift += 2.0 * ((p.cx[q] - p.cxf[q]) + (p.cy[q] - p.cyf[q]) + (p.cz[q] - p.czf[q]));
   }
   p.union_mask = 0;
   for (size_t t = 0; t < s.types.size(); t++) {

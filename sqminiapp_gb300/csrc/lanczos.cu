@@ -28,10 +28,10 @@ __global__ void veff_extend_kernel(const double *__restrict__ veff, double vcons
   }
 }
 
-// Quad-aligned copies of cdiag + Veff for the split-pass kernel: copy c holds extended x index
+// Quad-aligned copies of Veff for the split-pass kernel: copy c holds extended x index
 // ex at row position ex + c, so a node at grid x = I reads its cube row from copy (4 - I%4)%4
 // at a 16-byte boundary; positions outside [c, c + EX) hold 0.
-__global__ void veff_quad_kernel(const double *__restrict__ veff, double vconst, double cdiag,
+__global__ void veff_quad_kernel(const double *__restrict__ veff, double vconst,
                                  float *__restrict__ out, int Nx, int Ny, int Nz, int nhx, int nhy,
                                  int nhz, int EX, int EY, int EZ, int row) {
   const long long per_copy = (long long)row * EY * EZ;
@@ -49,7 +49,7 @@ __global__ void veff_quad_kernel(const double *__restrict__ veff, double vconst,
       const int gx = ((ex - nhx) % Nx + Nx) % Nx;
       const int gy = ((ey - nhy) % Ny + Ny) % Ny;
       const int gz = ((ez - nhz) % Nz + Nz) % Nz;
-      v = float(cdiag + (veff ? veff[((long long)gz * Ny + gy) * Nx + gx] : vconst));
+      v = float(veff ? veff[((long long)gz * Ny + gy) * Nx + gx] : vconst);
     }
     out[e] = v;
   }
@@ -179,13 +179,8 @@ cudaError_t launch_veff_extend(const double *veff, double vconst, void *ext, int
     const long long total = (long long)veff_quad_floats(p);
     const int block = 256;
     const int grid = (int)std::min<long long>((total + block - 1) / block, 152LL * 16);
-    // the diagonal also takes up what the FP32 stencil weights lose on a constant vector, so
-    // that their rounding does not shift the low end of the spectrum
-    double diag = p.cdiag;
-    for (int d = 1; d <= kStencilHalf; d++)
-      diag += 2.0 * ((p.cx[d] - p.cxf[d]) + (p.cy[d] - p.cyf[d]) + (p.cz[d] - p.czf[d]));
-    veff_quad_kernel<<<grid, block, 0, s>>>(veff, vconst, diag, (float *)ext, p.Nx, p.Ny, p.Nz,
-                                            p.nhx, p.nhy, p.nhz, p.EX, p.EY, p.EZ, p.vq_row);
+    veff_quad_kernel<<<grid, block, 0, s>>>(veff, vconst, (float *)ext, p.Nx, p.Ny, p.Nz, p.nhx,
+                                            p.nhy, p.nhz, p.EX, p.EY, p.EZ, p.vq_row);
     return cudaGetLastError();
   }
   const long long total = (long long)p.EX * p.EY * p.EZ;

@@ -15,9 +15,9 @@
 // Stencil, split by axis so that two of the three axes come from registers:
 //   pass A  a thread owns one quad (x..x+3) of row y over a z-range and walks z with a
 //           13-plane register ring (one float4 load per plane); the x neighbours of the quad
-//           are four aligned float4 loads of the same row; it adds the diagonal (cdiag + Veff,
-//           read as one aligned float4 from a quad-aligned copy of the padded potential) and
-//           forms U <- s (diag + Dz + Dx) P - gamma U;
+//           are four aligned float4 loads of the same row; it adds the diagonal (Veff, read as
+//           one aligned float4 from a quad-aligned copy of the padded potential; the stencil's
+//           own diagonal is left out, see Scaling) and forms U <- s (Veff + Dz + Dx) P - gamma U;
 //   pass B  a thread owns one quad of plane z over a y-range and walks y with a 13-row
 //           register ring: U += s Dy P.
 // Consecutive threads own consecutive quads in pass A; pass B's columns are dealt to the lanes by the
@@ -55,7 +55,11 @@
 // with a_k and gamma_k as double-floats (head and tail applied).  Normalising by a rounded 1/b_k left
 // |v_k| off by 1e-7 and so a_k by twice that of its 18 + V: that, not the stencil's rounding, was
 // most of the FP32 error (weights 6e-6 -> 4e-7 and the lowest Ritz value 5e-7 -> 5e-8 Ha on a 27^3
-// cube without projectors, the diagonal's share of the weights' rounding included).
+// cube without projectors).  What was left came from the stencil's constant diagonal (18 at h = 0.5,
+// where Veff is below 1): the start vector's H v and its a_0 were rounded at that size.  The recurrence
+// runs on H - hshift, which has the same vectors, b_k and weights, and hshift is added to a_k in FP64.
+// Restated on the CPU, 144 nodes of 27^3 and 40 steps: relative error of a node's weights 1.1e-6 -> 2.3e-7
+// (root mean square), 2.6e-6 -> 5.6e-7 (largest), at no cost.
 //
 // Memory traffic.  Pass A reads Veff from L2 one plane ahead.  Nodes after the first round come
 // from a device-side queue.
@@ -1009,7 +1013,7 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
     }
     __syncthreads();
 
-    // quad-aligned copy of the padded Veff + cdiag for this node (copy s: I + s = 0 mod 4)
+    // quad-aligned copy of the padded Veff for this node (copy s: I + s = 0 mod 4)
     const int sh = (4 - (I & 3)) & 3;
     const float4 *vq = reinterpret_cast<const float4 *>(veffq + (size_t)sh * p.vq_copy_stride) +
                        (size_t)((I + sh) >> 2);
@@ -1378,7 +1382,7 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
         if (r < steps) {
           const float2 one = make_float2(1.f, 0.f), np = r ? sum_b[r - 1] : one;
           const double n = (double)np.x + np.y;
-          av = ((double)sum_a[r].x + sum_a[r].y) / n;
+          av = ((double)sum_a[r].x + sum_a[r].y) / n + p.hshift;
           bv = sqrt(((double)sum_b[r].x + sum_b[r].y) / n) / (double)(r ? unit_scale(np.x) : 1.f);
         }
         double *o = ab_out + (node - p.node_begin) * 2 * p.nqp;

@@ -81,6 +81,7 @@ struct LanczosParams {
   double hx, hy, hz;
   float hxf, hyf, hzf;
   double cdiag;            // coeffs_x[0] + coeffs_y[0] + coeffs_z[0]
+  double hshift;           // kLayoutQuad: the kernel iterates on H - hshift and adds it to every a_k
   double cx[kStencilHalf + 1], cy[kStencilHalf + 1], cz[kStencilHalf + 1];
   float cdiagf;            // FP32 copies for the FP32 engine
   float cxf[kStencilHalf + 1], cyf[kStencilHalf + 1], czf[kStencilHalf + 1];

@@ -56,7 +56,7 @@ cudaError_t launch_lanczos(const LanczosParams &p, int precision, bool faithful,
 cudaError_t launch_veff_extend(const double *veff, double vconst, void *ext, int precision,
                                const LanczosParams &p, cudaStream_t s);
 
-// kLayoutQuad: the four quad-aligned copies of cdiag + Veff padded periodically by the cube
+// kLayoutQuad: the four quad-aligned copies of Veff padded periodically by the cube
 // half-width (copy s holds extended x index ex at row position ex + s; rows of vq_row floats).
 size_t veff_quad_floats(const LanczosParams &p);
 size_t lanczos_quad_smem_bytes(const LanczosParams &p);
