@@ -169,6 +169,7 @@ bool quad_list_bounds(const sq::Setup &s, const sq::Deck &d, sq::LanczosParams &
     const int z0 = ends[r], planes = ends[r + 1] - ends[r];
     if (planes == 0) continue;
     const int chunks = sq::lanczos_quad_list_chunks(columns, planes, block);
+    if ((planes + chunks - 1) / chunks > sq::kQuadListPlanes) return false;
     units = std::max(units, max_image_sum_per_node(s, d, [&](int a, int lo, int hi) {
       if (a == 0) return (hi >> 2) - (lo >> 2) + 1;
       if (a == 1) return hi - lo + 1;

@@ -332,8 +332,10 @@ template <int N> __device__ __forceinline__ void tmem_wait_ld(float4 (&t)[N][4],
       asm volatile("" : "+f"(t[c][i].x), "+f"(t[c][i].y), "+f"(t[c][i].z), "+f"(t[c][i].w));
 }
 
-// A unit's word: atom slot (10 bits), first plane from the first owned one (6), place of its partial
-// sums (16).
+// A unit's word: atom slot (10 bits), first plane from its item's first one (6), place of its partial
+// sums (16).  The host plans no list with longer items (kQuadListPlanes): from the cube's first plane the
+// field would end at 67 planes, and a cube of 17 x 17 x 69 points fits the SM.
+static_assert(kQuadListPlanes <= 63 + kRun, "6 bits hold the last unit's first plane");
 __device__ __forceinline__ unsigned unit_word(int slot, int z0, int place) {
   return (unsigned)(slot | (z0 << 10)) | ((unsigned)place << 16);
 }
@@ -801,7 +803,8 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
         int total = 0;  // of image k
         auto keep = [&](int k, ListRun r, int place) {
           if (!r.units()) return;
-          runs[(size_t)blockDim.x * n_run++] = make_int2(k | (r.a << 10) | (r.b << 17), place);
+          // planes from the item's first one, as in unit_word
+          runs[(size_t)blockDim.x * n_run++] = make_int2(k | ((r.a - it.zb) << 10) | ((r.b - it.zb) << 17), place);
           units += r.units();
         };
         for (unsigned todo = __ballot_sync(0xffffffffu, near); todo;) {  // two images at once
@@ -918,11 +921,11 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
       ImgRow g{};
       int i = 0;
       auto unit = [&](int u, float4 (&T)[NCH][kRun], float4 &meta) {
-        meta = make_float4(__uint_as_float(unit_word(0, item.zb, 0)), 0.f, 0.f, 0.f);
+        meta = make_float4(__uint_as_float(unit_word(0, 0, 0)), 0.f, 0.f, 0.f);
         const bool on = u < units;
         if (on && left == 0) {
           const int2 r = mine[(size_t)blockDim.x * i++];
-          const ListRun run{(r.x >> 10) & 127, r.x >> 17};
+          const ListRun run{item.zb + ((r.x >> 10) & 127), item.zb + (r.x >> 17)};
           a = run.a;
           b = run.b;
           left = run.units();
@@ -936,7 +939,7 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
         }
         const int z0 = on ? min(a, item.top - kRun) : item.zb;
         if (on)
-          meta = make_float4(__uint_as_float(unit_word(g.slot(), z0, place)), fmaf(p.hxf, item.x - g.bx, g.ox),
+          meta = make_float4(__uint_as_float(unit_word(g.slot(), z0 - item.zb, place)), fmaf(p.hxf, item.x - g.bx, g.ox),
                              fmaf(p.hyf, item.y - g.by, g.oy), fmaf(p.hzf, float(z0) - g.bz, g.oz));
         const float4 *tz = tq + (z0 - (int)g.bz) * nc;
         int c = 0, ch = 0;
@@ -1001,8 +1004,8 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
           for (int q = 0; q < kRun; q++) T[c][q] = wT[((u * NCH + c) * kRun + q) * 32];
       }
     };
-    // the item's column in P (owned planes) and U
-    const unsigned itemP = 16u * (unsigned)(item.column + (zo0 - pz0) * PS4), itemU = 16u * (unsigned)item.column;
+    // the item's first quad in P and U
+    const unsigned itemU = 16u * (unsigned)(item.column + item.zb * PS4), itemP = itemU + (unsigned)((zo0 - pz0) * PB);
     unsigned aP0 = sP, aU0 = sU;  // the arrays of P and U (kSwap: they change places every step)
     __syncthreads();  // the scratch in U is read
     for (int e = threadIdx.x; e < (ncu >> 2); e += blockDim.x) U4[e] = zero4;

@@ -67,6 +67,7 @@ int lanczos_quad_block(const LanczosParams &p);
 // of one CTA's slice of global scratch; and room in shared memory for the units' partial sums (part_cap)
 // with the CTAs that share an SM (returned) and their tensor-memory columns (list_columns).
 constexpr int kQuadListRun = 4;
+constexpr int kQuadListPlanes = 67;  // the longest plane range whose units the list's words hold
 int lanczos_quad_list_chunks(int columns, int planes, int threads);
 size_t lanczos_quad_unit_bytes(const LanczosParams &p);
 size_t lanczos_quad_list_bytes(const LanczosParams &p);
