@@ -1060,9 +1060,11 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
         }
         const float4 *vrow = vq + (size_t)(K * p.EY + J + yA) * VRS4 + ql + (size_t)zbA * VPS4;
         // the quad at plane zbA + i of P and U, and P's plane 6 further on: all lanes make zlen
-        // steps (a uniform loop), those past their range keep nothing
-        unsigned aP = aP0 + 16u * (unsigned)(row4 + zbA * PS4 + pofs4);
-        unsigned aN = aP + (unsigned)(O * PB);
+        // steps (a uniform loop), those past their range keep nothing and read the x neighbours (aX) of
+        // their last plane again: the planes after it may lie beyond P, whose place behind U with
+        // kSwap has no array of that size after it
+        const unsigned aP = aP0 + 16u * (unsigned)(row4 + zbA * PS4 + pofs4);
+        unsigned aX = aP, aN = aP + (unsigned)(O * PB);
         unsigned aU = aU0 + 16u * (unsigned)(row4 + zbA * PS4 + uofs4);
         const int live = zeA - zbA, above = nz - O - zbA;
         float4 ring[W];
@@ -1085,13 +1087,14 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
             if (i >= zlen) break;
             ring[s] = lds_quad(i < above ? aN : sZ);
 #define RING(dd) ring[(s + (dd) + O + 1) % W]
-            lds_pair_if<-24>(hm2, aP, xm2);
-            lds_quad_if<-16>(hm1, aP, xm1);
-            lds_quad_if<16>(hp1, aP, xp1);
-            lds_pair_if<32>(hp2, aP, xp2);
+            lds_pair_if<-24>(hm2, aX, xm2);
+            lds_quad_if<-16>(hm1, aX, xm1);
+            lds_quad_if<16>(hp1, aX, xp1);
+            lds_pair_if<32>(hp2, aX, xp2);
             const float4 c = RING(0);
             const float4 dv = dv1, uo = lds_quad(i < live ? aU : sZ);
-            dv1 = __ldg(vrow + min(i + 1, live - 1) * VPS4);
+            const int next = min(i + 1, live - 1);
+            dv1 = __ldg(vrow + next * VPS4);
             float2 h01 = mul2(lo(dv), lo(c)), h23 = mul2(hi(dv), hi(c));
 #pragma unroll
             for (int d = 1; d <= O; d++) {
@@ -1121,7 +1124,7 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
             sts_quad_if(i < live, aU, make_float4(n01.x, n01.y, n23.x, n23.y));
             const float2 pa = fma2(lo(c), h01, mul2(hi(c), h23));
             ka.add(i < live ? pa.x + pa.y : 0.f);
-            aP += (unsigned)PB;
+            aX = aP + (unsigned)(next * PB);
             aN += (unsigned)PB;
             aU += (unsigned)PB;
           }
