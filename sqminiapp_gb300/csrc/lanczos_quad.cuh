@@ -322,6 +322,13 @@ __device__ __forceinline__ void tmem_st4(unsigned taddr, float4 a) {
 __device__ __forceinline__ void tmem_wait_st() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
+// A barrier of the CTA that also orders the tensor-memory accesses of its warps: a warp's units have other
+// places in the next node, where another warp of the same lanes read before.
+__device__ __forceinline__ void tmem_sync() {
+  tc5::fence_before_sync();
+  __syncthreads();
+  tc5::fence_after_sync();
+}
 // The wait names the registers it guards, so that no use of them moves above it.
 template <int N> __device__ __forceinline__ void tmem_wait_ld(float4 (&t)[N][4], float4 &m) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" : "+f"(m.x), "+f"(m.y), "+f"(m.z), "+f"(m.w)::"memory");
@@ -645,7 +652,7 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
   // list items: column (quad xq of row y) and plane range [nzo c / nlc, nzo (c+1) / nlc) of the owned
   const int ncol = nq * ny, nlc = list_chunks(ncol, nzo, blockDim.x), n_item = ncol * nlc;
   if (warp == 0) tc5::tmem_alloc(reinterpret_cast<uint32_t *>(cnt + 4), (uint32_t)p.list_columns);
-  __syncthreads();
+  tmem_sync();
   const float ihz = 1.f / p.hzf;
   const unsigned tquarter = (unsigned)cnt[4] + ((unsigned)(warp & 3) << 21);  // the warp's lanes
 
@@ -1395,7 +1402,8 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
         o[r] = av;
         o[p.nqp + r] = bv;
       }
-    __syncthreads();
+    // the next node's units (or the release below) take the places that this node's warps read
+    tmem_sync();
   }
   // no CTA of a pair leaves while its peer may still read its shared memory
   if constexpr (PAIR) cooperative_groups::this_cluster().sync();
