@@ -554,18 +554,20 @@ void build_engine(sq_handle *h) {
   const sq::Setup &s = h->setup;
   const sq::LanczosParams &p = h->lp;
 
-  // device buffers
+  // device buffers, filled in the handle's stream: use_quad_tables reads them there, and a copy in the
+  // default stream may still be on its way when cudaMemcpy returns (pageable memory)
   dev_alloc(&h->d_images, sizeof(sq::ImageMeta) * s.images.size(), "images");
-  ck(cudaMemcpy(h->d_images, s.images.data(), sizeof(sq::ImageMeta) * s.images.size(),
-                cudaMemcpyHostToDevice), "images H2D");
+  ck(cudaMemcpyAsync(h->d_images, s.images.data(), sizeof(sq::ImageMeta) * s.images.size(),
+                     cudaMemcpyHostToDevice, h->own_stream), "images H2D");
   dev_alloc(&h->d_tables, h->elem * s.tables.size(), "tables");
   if (h->opt.precision == 32) {
     std::vector<float> t32(s.tables.begin(), s.tables.end());
-    ck(cudaMemcpy(h->d_tables, t32.data(), 4 * t32.size(), cudaMemcpyHostToDevice), "tables H2D");
+    ck(cudaMemcpyAsync(h->d_tables, t32.data(), 4 * t32.size(), cudaMemcpyHostToDevice, h->own_stream),
+       "tables H2D");
     if (h->quad) use_quad_tables(h);
   } else {
-    ck(cudaMemcpy(h->d_tables, s.tables.data(), 8 * s.tables.size(), cudaMemcpyHostToDevice),
-       "tables H2D");
+    ck(cudaMemcpyAsync(h->d_tables, s.tables.data(), 8 * s.tables.size(), cudaMemcpyHostToDevice,
+                       h->own_stream), "tables H2D");
   }
   dev_alloc(&h->d_veff_ext,
             h->quad ? sizeof(float) * sq::veff_quad_floats(p) : h->elem * (size_t)p.EX * p.EY * p.EZ,
@@ -577,12 +579,13 @@ void build_engine(sq_handle *h) {
   }
   dev_alloc(&h->d_proj, (size_t)p.proj_bytes_per_cta * h->grid, "projector list scratch");
   dev_alloc(&h->d_status, sizeof(int) * 4, "status");
-  ck(cudaMemset(h->d_status, 0, sizeof(int) * 4), "status memset");
+  ck(cudaMemsetAsync(h->d_status, 0, sizeof(int) * 4, h->own_stream), "status memset");
   h->fermi_grid = h->num_sms;
   dev_alloc(&h->d_fermi_scratch, sizeof(double) * sq::fermi_scratch_doubles(h->fermi_grid, h->fermi_maxit),
             "fermi scratch");
   dev_alloc(&h->d_bar, sizeof(unsigned) * 2, "barrier");
   dev_alloc(&h->d_fermi_out, sizeof(double) * 4, "fermi out");
+  ck(cudaStreamSynchronize(h->own_stream), "engine buffers");
 }
 
 }  // namespace
