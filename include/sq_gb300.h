@@ -170,6 +170,12 @@ sq_status sq_get_info(const sq_handle *h, sq_info *info);
 sq_status sq_plan_kernel(const char *deck_dir, const char *name, const sq_options *opt,
                          int num_sms, int smem_optin, int l2_bytes, sq_info *info);
 
+/* Host-only plan of a batch (no GPU touched): the SMs that sq_batch_nodes_and_weights gives each of
+ * n_cells cells of n_nodes[c] nodes that cost node_cost[c] on one SM (any unit) and run ctas_per_sm[c] CTAs,
+ * of one node each, on an SM. */
+sq_status sq_plan_batch(const double *node_cost, const long *n_nodes, const int *ctas_per_sm, int n_cells,
+                        int num_sms, int *sms);
+
 /* Per-node Lanczos + Gauss quadrature for nodes [node_begin, node_end) in the reference's
  * node order (z slowest, x fastest; src/lsdft_scf.cc:60-67).  Replaces
  * NodesAndWeights_LSSGQ (src/lsdft.h:132, called at src/main.cc:54), which loops

@@ -635,7 +635,7 @@ void update_node_cost(sq_handle *h) {
 
 sq_status run_device(sq_handle *h, const double *d_veff, double veff_const, long long nb,
                      long long ne, double *d_lambda, double *d_w, double *d_lmin, double *d_lmax,
-                     cudaStream_t s, int grid_limit) {
+                     cudaStream_t s, int sm_limit) {
   const long long n = ne - nb;
   if (nb < 0 || ne > h->info.n_nodes || n <= 0)
     return fail(SQ_BAD_INPUT, "node range outside the grid");
@@ -645,16 +645,17 @@ sq_status run_device(sq_handle *h, const double *d_veff, double veff_const, long
   p.node_end = ne;
   ck(cudaMemsetAsync(h->d_status, 0, sizeof(int), s), "status reset");
   ck(sq::launch_veff_extend(d_veff, veff_const, h->d_veff_ext, h->opt.precision, p, s), "veff");
-  int grid = (int)std::min<long long>(grid_limit > 0 ? std::min(grid_limit, h->grid) : h->grid, n);
+  const int ctas = sm_limit > 0 ? std::min(sm_limit * h->quad_ctas, h->grid) : h->grid;
+  int grid = (int)std::min<long long>(ctas, n);
   if (p.layout & sq::kLayoutPair)  // two CTAs per node: an even grid, one pair per node at most
-    grid = 2 * (int)std::max<long long>(
-                   1, std::min<long long>((grid_limit > 0 ? std::min(grid_limit, h->grid) : h->grid) / 2, n));
+    grid = 2 * (int)std::max<long long>(1, std::min<long long>(ctas / 2, n));
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   ck(cudaStreamIsCapturing(s, &cap), "capture status");
   const bool timed = cap == cudaStreamCaptureStatusNone;  // no timing events inside a graph
   if (timed) {
     update_node_cost(h);
-    h->cost_grid = grid_limit > 0 ? grid : std::max(1, grid / h->quad_ctas);  // SMs
+    // SMs at work: CTAs go to idle SMs first
+    h->cost_grid = std::min(grid, sm_limit > 0 ? sm_limit : h->num_sms);
     h->cost_nodes = n;
     ck(cudaEventRecord(h->ev[0], s), "event");
   }
@@ -675,6 +676,23 @@ sq_status run_device(sq_handle *h, const double *d_veff, double veff_const, long
 }  // namespace sq
 
 namespace {
+// SMs of every cell of a batch: one each, then every further SM to the cell that would finish last.  A
+// cell's finish counts whole rounds of nodes, one per CTA: with k CTAs on an SM a round takes k times
+// the cost of a node on one SM.
+void split_sms(const double *cost, const long *nodes, const int *ctas, int n_cells, int sms, int *share) {
+  std::fill(share, share + n_cells, 1);
+  auto finish = [&](int c) {
+    return std::ceil((double)nodes[c] / ((double)share[c] * ctas[c])) * ctas[c] * cost[c];
+  };
+  for (int left = sms - n_cells; left > 0; left--) {
+    int worst = 0;
+    for (int c = 1; c < n_cells; c++)
+      if (finish(c) > finish(worst)) worst = c;
+    if (share[worst] >= nodes[worst]) break;  // more SMs would idle
+    share[worst]++;
+  }
+}
+
 sq_status describe(const sq::Deck &d, int faithful, sq_info *info, double *gamma, double *cutoff) {
   sq::Setup s = sq::build_setup(d, faithful != 0);
   sq_options opt{faithful, 0, 0, 0, 0, 0};
@@ -952,6 +970,19 @@ sq_status sq_measure_fp32_peak(int device, double *tflops) {
   });
 }
 
+sq_status sq_plan_batch(const double *node_cost, const long *n_nodes, const int *ctas_per_sm, int n_cells,
+                        int num_sms, int *sms) {
+  if (!node_cost || !n_nodes || !ctas_per_sm || !sms) return fail(SQ_BAD_INPUT, "null argument");
+  if (n_cells <= 0 || n_cells > num_sms) return fail(SQ_BAD_INPUT, "1 to num_sms cells");
+  for (int c = 0; c < n_cells; c++)
+    if (!(node_cost[c] > 0.0) || n_nodes[c] <= 0 || ctas_per_sm[c] <= 0)
+      return fail(SQ_BAD_INPUT, "costs, nodes and CTAs must be positive");
+  return guarded([&] {
+    split_sms(node_cost, n_nodes, ctas_per_sm, n_cells, num_sms, sms);
+    return SQ_OK;
+  });
+}
+
 sq_status sq_batch_nodes_and_weights(sq_handle *const *cells, int n_cells, const double *const *d_veff,
                                      const double *veff_const, double *const *d_lambda,
                                      double *const *d_weights, double *const *d_lambda_min,
@@ -985,28 +1016,26 @@ sq_status sq_batch_nodes_and_weights(sq_handle *const *cells, int n_cells, const
                              : in.n_qp * ((2.0 * (6 * in.fd_half_order + 1) + 9.0) * nc +
                                           4.0 * in.n_lm * in.proj_points_per_node);
     }
-    // one SM each, then every further SM to the cell that would finish last; a cell's finish
-    // time counts whole rounds of nodes, ceil(nodes / SMs) x cost per node
-    std::vector<int> share(n_cells, 1);
-    auto finish = [&](int c, int sh) {
-      return std::ceil((double)cells[c]->info.n_nodes / sh) * per_node[c];
-    };
-    for (int left = sms - n_cells; left > 0; left--) {
-      int worst = 0;
-      for (int c = 1; c < n_cells; c++)
-        if (finish(c, share[c]) > finish(worst, share[worst])) worst = c;
-      if (share[worst] >= cells[worst]->info.n_nodes) break;  // more SMs would idle
-      share[worst]++;
+    std::vector<long> nodes(n_cells);
+    std::vector<int> ctas(n_cells), share(n_cells), order(n_cells);
+    for (int c = 0; c < n_cells; c++) {
+      nodes[c] = cells[c]->info.n_nodes;
+      ctas[c] = cells[c]->quad_ctas;
+      order[c] = c;
     }
+    split_sms(per_node.data(), nodes.data(), ctas.data(), n_cells, sms, share.data());
     // fork: every cell's stream waits for the caller's stream and runs its cell on its SM
-    // share; the caller's stream waits for all of them
+    // share; the caller's stream waits for all of them.  Cells with a whole SM per CTA first: CTAs
+    // that share SMs go to idle ones first, and would leave no whole one.
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return ctas[a] < ctas[b]; });
     cudaStream_t s = (cudaStream_t)stream;
     cudaEvent_t fork = nullptr;
     ck(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming), "event");
     std::vector<cudaEvent_t> join(n_cells, nullptr);
     sq_status st = SQ_OK;
     ck(cudaEventRecord(fork, s), "event");
-    for (int c = 0; c < n_cells && st == SQ_OK; c++) {
+    for (int i = 0; i < n_cells && st == SQ_OK; i++) {
+      const int c = order[i];
       sq_handle *h = cells[c];
       ck(cudaStreamWaitEvent(h->own_stream, fork, 0), "wait");
       st = run_device(h, d_veff ? d_veff[c] : nullptr, veff_const ? veff_const[c] : 0.0, 0,

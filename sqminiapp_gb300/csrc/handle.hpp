@@ -112,10 +112,10 @@ struct sq_handle {
 namespace sq {
 
 // Per-node Lanczos + quadrature of nodes [nb, ne) on stream s (device buffers).
-// grid_limit > 0 caps the persistent grid (CTAs = SMs used), else one CTA per SM.
+// sm_limit > 0 caps the SMs that the persistent grid fills (quad_ctas CTAs each), else all of them.
 sq_status run_device(sq_handle *h, const double *d_veff, double veff_const, long long nb,
                      long long ne, double *d_lambda, double *d_w, double *d_lmin, double *d_lmax,
-                     cudaStream_t s, int grid_limit = 0);
+                     cudaStream_t s, int sm_limit = 0);
 // Folds the timing of the last Lanczos launch, once its events have completed, into
 // node_sm_ms (non-blocking).
 void update_node_cost(sq_handle *h);
