@@ -221,12 +221,13 @@ __global__ void __launch_bounds__(kFermiBlock)
   const double inv_beta = 1.0 / beta;
 
   // phase 1a: kFermiLevels levels per pass in FP32.  Of a level's sum S the rounding of lambda (1e-7
-  // of |lambda|, beta times that of the exponent) and of the float sums stay below err S.
+  // of |lambda|, beta times that of the exponent), of the terms and of the float sums (2^-24 of S for
+  // each term that a thread adds) stay below err S.
   if (!plain) {
     double cl = lo, cr = hi;
     const float bf = (float)beta;
     const double span = fmax(fabs(lo), fabs(hi));
-    const double err = 1e-4 + 4e-7 * beta * span;
+    const double err = 1e-4 + 4e-7 * beta * span + 6e-8 * (double)((n + stride - 1) / stride);
     for (int pass = 0; pass < 24 && cr - cl > 0.25 * inv_beta && err < 0.25; pass++) {
       float lev[kFermiLevels], c[kFermiLevels];
 #pragma unroll
