@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(kFermiBlock)
     for (int q = 0; q < nqp; q++) {
       const long long e = node * nqp + q;
       const double l = lambda[e], x = beta * (l - lf);
-      if (x > 745.2) continue;  // empty
+      if (x > 745.2 && !plain) continue;  // empty (an infinite weight times 0 has to reach the sums)
       const double f = fermi_dirac(beta, l, lf);
       r += w[e] * f;
       eb += 2.0 * w[e] * l * f;
