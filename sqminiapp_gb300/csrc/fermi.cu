@@ -108,9 +108,11 @@ __device__ __forceinline__ float truncate_f32(double v) {
 }
 
 // In units of 1/beta: entries this far above a level count as empty in the gathered sums (their
-// occupation is below 2e-20, under half an ulp of any sum that holds a single state), and this far
-// below as full (exactly 1 in FP64).
+// occupation is below 2e-20, 2e-13 of the electrons if all states of a cell that is filled to kFermiLeast
+// lie there), and this far below as full (exactly 1 in FP64).
 constexpr double kFermiAbove = 45.5, kFermiBelow = 37.5;
+// With a smaller share of the states filled every midpoint is summed over all entries.
+constexpr double kFermiLeast = 1e-7;
 constexpr int kFermiLevels = 3;    // levels per FP32 pass
 constexpr int kFermiRows = 2 * kFermiLevels + 2;  // scratch rows: partials of two passes, bracket
 constexpr int kFermiEntries = 4096;  // entries of a CTA's slice gathered in shared memory
@@ -154,8 +156,9 @@ __global__ void __launch_bounds__(kFermiBlock)
   double *bracket = scratch + (long long)(2 * kFermiLevels) * G;
   int parity = 0;  // which half of the partial rows the next pass writes
 
-  // phase 0: bracket, and whether N_e is known to grow with the level
+  // phase 0: bracket, the weights' sum, and whether N_e is known to grow with the level
   double lo = 1e300, hi = -1e300;
+  float filled = 0.f;
   bool plain = false;
   for (long long e = tid; e < n; e += stride) {
     const double l = lambda[e];
@@ -164,7 +167,9 @@ __global__ void __launch_bounds__(kFermiBlock)
     // a weight below zero or not finite, a value not finite (exponent all ones)
     const int wh = __double2hiint(w[e]), lh = __double2hiint(l);
     plain = plain || (wh < 0 && (wh & 0x7fffffff)) || ((wh >> 20) & 2047) == 2047 || ((lh >> 20) & 2047) == 2047;
+    filled += truncate_f32(w[e]);
   }
+  const double filled_all = block_sum_d(2.0 * (double)filled, red);  // in thread 0
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
@@ -186,26 +191,31 @@ __global__ void __launch_bounds__(kFermiBlock)
     for (int i = 1; i < kFermiBlock / 32; i++) m = fmax(m, red[i]);
     bracket[G + blockIdx.x] = m;
     scratch[blockIdx.x] = plain ? 1.0 : 0.0;
+    scratch[G + blockIdx.x] = filled_all;
   }
   if (!grid_barrier(bar, status, &flag, spin_limit)) return;
   {
-    double a = 1e300, b = -1e300, q = 0.0;
+    double a = 1e300, b = -1e300, q = 0.0, t = 0.0;
     if (threadIdx.x < 32) {
       for (int i = threadIdx.x; i < G; i += 32) {
         a = fmin(a, __ldcg(bracket + i));
         b = fmax(b, __ldcg(bracket + G + i));
         q += __ldcg(scratch + i);
+        t += __ldcg(scratch + G + i);
       }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
         a = fmin(a, __shfl_xor_sync(0xffffffffu, a, o));
         b = fmax(b, __shfl_xor_sync(0xffffffffu, b, o));
         q += __shfl_xor_sync(0xffffffffu, q, o);
+        t += __shfl_xor_sync(0xffffffffu, t, o);
       }
       if (threadIdx.x == 0) {
         bcast[0] = a - 1.0;
         bcast[1] = b + 1.0;
-        bcast[2] = q;
+        // nearly empty: the electrons are no longer far more than what the gathered sums leave out
+        // (kFermiAbove) and the FP32 passes cap (exponents above 80); or weights outside FP32's range
+        bcast[2] = q != 0.0 || !(n_electrons >= kFermiLeast * t) || !(t > 1e-25);
       }
     }
     __syncthreads();
