@@ -116,8 +116,8 @@ __global__ void __launch_bounds__(kQuadBlock)
       do {
         for (m = l; m <= nqp - 2; m++) {
           const double em = e[m], dm = d[m], dn = d[m + 1];
-          const int xe = exponent(em);
-          if (xe > 0 && xe >= max(exponent(dm), exponent(dn)) - 51) continue;  // |e| > 2^-53 dd
+          const int xe = exponent(em), xd = max(exponent(dm), exponent(dn));
+          if (xe > 0 && xe >= xd - 51 && xd < 2046) continue;  // |e| > 2^-53 dd, and dd does not overflow
           const double dd = fabs(dm) + fabs(dn);
           if (fabs(em) + dd == dd) break;
         }
