@@ -19,7 +19,15 @@ int lanczos_quad_threads(const LanczosParams &p) {
 int lanczos_quad_block(const LanczosParams &p) {
   // every warp of the register budget (12 warps at up to 384 threads, 16 above): the passes
   // use lanczos_quad_threads of them, the list streams and the update all
-  const int t = lanczos_quad_threads(p);
+  int t = lanczos_quad_threads(p);
+  // at least as many as give the list items that its words hold (a cube of 3 x 69 x 69 points and one
+  // range has a thread per column, of 69 planes)
+  const int columns = p.pitch / 4 * p.ny;
+  auto longest = [&](int threads) {
+    const int chunks = lq::list_chunks(columns, p.nz, threads);
+    return (p.nz + chunks - 1) / chunks;
+  };
+  while (t < kQuadMaxThreads && longest(t) > kQuadListPlanes) t += 32;
   if (t <= 256) return t;
   return t <= 384 ? 384 : kQuadMaxThreads;
 }

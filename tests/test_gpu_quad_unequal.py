@@ -19,6 +19,8 @@ CASES = [((12, 12, 54), 5.2, 10, 2, (17, 17, 69), 16), ((10, 10, 60), 5.2, 10, 1
          ((13, 13, 66), 5.0, 10, 0, (17, 17, 79), 16), ((6, 6, 120), 4.2, 10, 2, (7, 7, 121), 16),
          ((15, 15, 60), 5.6, 8, 2, (21, 21, 81), 48), ((5, 60, 5), 4.2, 10, 1, (7, 61, 7), 16),
          ((13, 17, 15), 5.0, 10, 0, (17, 21, 19), 16), ((18, 16, 14), 4.5, 10, 2, (21, 19, 17), 16)]
+# with one range per row: a thread per column would own 69 planes
+ONE_RANGE = ((2, 68, 68), 4.2, 8, 2, (3, 69, 69), 16)
 
 
 def _deck(path, grid, rcut, q, lloc):
@@ -35,10 +37,10 @@ def _list_chunks(columns, planes, threads):
     return c
 
 
-@pytest.mark.parametrize("grid,rcut,q,lloc,cube,layout", CASES)
-def test_plan_and_word_widths(grid, rcut, q, lloc, cube, layout, tmp_path):
+@pytest.mark.parametrize("grid,rcut,q,lloc,cube,layout,tile", [c + (0,) for c in CASES] + [ONE_RANGE + (1,)])
+def test_plan_and_word_widths(grid, rcut, q, lloc, cube, layout, tile, tmp_path):
     """CPU: the planned kernel, and a unit's first plane within 6 bits of its item's first one."""
-    info = plan_kernel(*_deck(tmp_path, grid, rcut, q, lloc))
+    info = plan_kernel(*_deck(tmp_path, grid, rcut, q, lloc), kernel=2, tile=tile)
     assert tuple(info.cube) == cube and info.kernel_layout == layout
     planes = cube[2] if layout == 16 else (cube[2] + 1) // 2
     columns = (cube[0] + 3) // 4 * cube[1]
@@ -50,15 +52,15 @@ def test_plan_and_word_widths(grid, rcut, q, lloc, cube, layout, tmp_path):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("grid,rcut,q,lloc,cube,layout", CASES)
-def test_against_oracle(grid, rcut, q, lloc, cube, layout, tmp_path, oracle_mod):
+@pytest.mark.parametrize("grid,rcut,q,lloc,cube,layout,tile", [c + (0,) for c in CASES] + [ONE_RANGE + (1,)])
+def test_against_oracle(grid, rcut, q, lloc, cube, layout, tile, tmp_path, oracle_mod):
     from sqminiapp_gb300 import LSDFT
     d, name = _deck(tmp_path, grid, rcut, q, lloc)
     o = oracle_mod.Oracle(d, name, faithful=False)
     nodes = np.arange(0, o.n_nodes, max(1, o.n_nodes // 11))
     veff = -0.3 + 0.1 * np.random.default_rng(q).standard_normal(o.n_nodes)
     ref = o.nodes_and_weights(nodes=nodes, veff=veff, want_ab=True)
-    with LSDFT(d, name, faithful=False, precision=32) as eng:
+    with LSDFT(d, name, faithful=False, precision=32, kernel=2, tile=tile) as eng:
         assert eng.cube == cube and eng.info.kernel_layout == layout
         out = eng.NodesAndWeights_LSSGQ(veff=veff)
         a, b = eng.lanczos_coefficients(eng.n_nodes)
