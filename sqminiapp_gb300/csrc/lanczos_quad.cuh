@@ -1131,7 +1131,10 @@ __device__ __forceinline__ void quad_body(const LanczosParams &p, const float *_
             sts_quad_if(i < live, aU, make_float4(n01.x, n01.y, n23.x, n23.y));
             const float2 pa = fma2(lo(c), h01, mul2(hi(c), h23));
             ka.add(i < live ? pa.x + pa.y : 0.f);
-            aX = aP + (unsigned)(next * PB);
+            // (a pair has one range, so all its lanes walk to their end together: the sum is 1% faster there,
+            // the product 0.5% in the others; 9001 nodes of 33^3 106.7 -> 105.6 ms, 39304 of 27^3 168.4 -> 167.5)
+            if constexpr (PAIR) aX += (unsigned)PB;
+            else aX = aP + (unsigned)(next * PB);
             aN += (unsigned)PB;
             aU += (unsigned)PB;
           }
